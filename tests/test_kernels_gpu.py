@@ -92,6 +92,26 @@ def test_gemm_f32_is_true_32_bit_and_batch_invariant(M, N, K):
     assert float((out.cpu().double() - want).abs().max()) <= 2e-6 * math.sqrt(K) * float(want.abs().max())
 
 
+@pytest.mark.parametrize("N, K", [(64, 32), (65, 1001), (896, 896), (130, 4864), (9728, 100), (2048, 1024), (38000, 36), (1, 3)])
+def test_gemm_f32_sums_do_not_hang_off_the_number_of_tokens(N, K):
+    """Every kernel and tile that the product chooses by the number of tokens, at the edges of the choice: the same bits."""
+    from easy_gpt.cpp_b200 import kernels
+
+    most = 640 if N < 4000 else 200
+    a, w, b = (torch.randn(*s, generator=gen(8 + i)) for i, s in enumerate(((most, K), (N, K), (N,))))
+    want = a.double() @ w.double().t() + b.double()
+    whole = torch.empty(most, N, device=DEV)
+    a, w, b = a.to(DEV), w.to(DEV), b.to(DEV)
+    kernels.gemm_f32_nt(a, w, b, whole)
+    # a K-term float32 sum in parts of at most K terms: 2e-6 sqrt(K) of the largest element, as for the sizes above
+    assert float((whole.cpu().double() - want).abs().max()) <= 2e-6 * math.sqrt(K) * float(want.abs().max())
+    for M in (1, 4, 5, 8, 9, 16, 17, 32, 33, 64, 65, 128, 129, most - 1):
+        first = most - M                                   # the last M rows: other tiles than in the whole
+        out = torch.empty(M, N, device=DEV)
+        kernels.gemm_f32_nt(a[first:], w, b, out)
+        assert torch.equal(out, whole[first:]), M
+
+
 # -- rotary encoding + cache write -----------------------------------------------------
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
