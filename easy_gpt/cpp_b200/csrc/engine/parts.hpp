@@ -127,7 +127,7 @@ public:
                                     x ? x->p : nullptr, x ? x->ld : 0, resid_in, resid_out, delta, gain, eps, out, ldo, plan.row_blocks,
                                     plan.k_slices, plan.k_split, partials, counters, r.num_heads, r.num_kv_heads, r.head_dim, r.positions,
                                     r.slot_map, r.k_cache, r.v_cache, r.inv_freq, r.page_size, r.page_stride, r.head_stride, r.pool_slots,
-                                    ctx.status, nullptr, 0, nullptr, ss_in, ss_parts, follow_residual, follow_gain, xn_out, ss_out),
+                                    ctx.status, epilogue == plans::EPI_RESID_NORM ? ctx.soon : nullptr, (long long)ctx.soon_bytes, nullptr, ss_in, ss_parts, follow_residual, follow_gain, xn_out, ss_out),
                      "gemm_skinny");
     }
 
@@ -807,6 +807,10 @@ public:
         return b.linear(d, down_.weight, inter_, down_.bias_f32(), nullptr);
     }
 
+    const void* first_weights(size_t* bytes) const override {
+        *bytes = gate_up_.weight_bytes();
+        return gate_up_.weight;
+    }
     Delta forward(const StepContext& ctx, PartInput in, const FollowingNorm* follow) override {
         const int T = ctx.num_tokens;
         const DType dtype = ctx.dtype;

@@ -136,6 +136,9 @@ struct StepContext {
     int num_tiles = 0;
     const int* small_tokens = nullptr;  // token indices of the entries too short for tiles
     int num_small = 0;
+    // weights that the sub-layer behind the current one reads first: a decode product with time to spare asks the L2 for them
+    const void* soon = nullptr;
+    size_t soon_bytes = 0;
     std::map<std::string, void*> shared;    // per-step data that parts share between layers (cleared at every forward)
 
     template <class T> T* take(size_t n) const { return arena->take_n<T>(n); }
@@ -468,6 +471,8 @@ public:
 class FeedForward : public Part {
 public:
     using Part::Part;
+    // the weights its first product streams (nullptr: unknown)
+    virtual const void* first_weights(size_t* /*bytes*/) const { return nullptr; }
     virtual bool accepts_pending_norm() const { return false; }
     virtual bool fuses_following_norm() const { return false; }
     virtual Delta forward(const StepContext& ctx, PartInput x, const FollowingNorm* follow) = 0;

@@ -1,5 +1,9 @@
 // Matrix products for decode steps (1..64 tokens): y[m, n] = sum_k x[m, k] W[n, k].
 //
+// The kernel of this file is register-fed; up to 16 tokens gemm_stream.cu takes the products whose rows need no add + norm
+// here (all but a step's first), and this one the rest: 17 to 64 tokens, the add + norm prologue, heads that are no multiple
+// of 32, residuals whose partial sums are asked for by larger groups of rows, K ranges whose clusters do not find room.
+//
 // With so few tokens the product is a stream of the weights from HBM, so the
 // kernel is built around that stream.  The roles of the MMA are swapped: 16 weight
 // rows are the M side of mma.m16n8k16 and 8 tokens are its N side, so no tensor
@@ -46,63 +50,15 @@
 // stream has been issued it asks the L2 (126 MB) to fetch them.
 #include <cstdlib>
 
+#include "gemm_skinny.cuh"
 #include "mma_utils.cuh"
 
 namespace {
+using namespace skinny;
 
 constexpr int MAX_THREADS = 512;
 constexpr int UNROLL = 4;            // 64-wide k chunks in flight per warp (256 bytes per thread)
 constexpr int CHUNK = 64;
-
-enum { EPI_STORE = 0, EPI_F32 = 1, EPI_SWIGLU = 2, EPI_QKV_ROPE = 3, EPI_RESID_NORM = 4 };
-
-struct Params {
-    const bf16* W;
-    long long ldw;
-    const float* bias;
-    int M, N, K;
-    const bf16* x;
-    long long ldx;
-    const float* resid_in;
-    float* resid_out;
-    const bf16* delta;
-    const float* gain;
-    float eps;
-    bf16* out;
-    long long ldo;
-    float* out_f32;
-    int num_heads, num_kv_heads, head_dim;
-    const int* positions;
-    const int* slot_map;
-    bf16* k_cache;
-    bf16* v_cache;
-    const float* inv_freq;
-    int page_size;
-    long long page_stride, head_stride, pool_slots;
-    int* status;
-    int RB, KS;
-    int use_pdl;
-    int stage_norm;              // the norm prologue's input comes through one bulk copy into shared memory
-    int norm_mode;               // 1: add + norm here; 2: prenormed rows (delta = xn) and partial sums (ss_in)
-    const float* ss_in;          // [ss_parts][padded tokens] partial sums of squares, prenormed prologue
-    int ss_parts;
-    float* resid_inout;          // resid_norm epilogue: the residual, updated in place
-    const float* gain_out;       //   the following norm's gain
-    bf16* xn_out;                //   bfloat16(gain_out * v) [M, N]
-    float* ss_out;               //   [gridDim.x][padded tokens]
-    // EPI_STORE with an activation on the way out: act 1: act(z) = act_a z^2 + z / 2 for z > 0, act_b (e^z - 1 - z) + z / 2
-    // below; act 2: act(z) = max(z, 0)^2; act 4: the exact gelu.  EPI_SWIGLU with act 3: g = min(gate, act_a), u = clamp(up, -act_a, act_a),
-    // out = g sigmoid(1.702 g) (u + 1)
-    int act;
-    float act_a, act_b;
-    const void* prefetch;        // weights of a kernel that runs soon: pulled into L2 meanwhile
-    long long prefetch_bytes;
-    float* scratch;              // [gridDim.y][gridDim.x][RB*16][tokens] partial sums when K is cut across CTAs
-    int* counters;               // [gridDim.x] tickets, zero before and after every launch
-    unsigned long long* trace;   // optional: [2] earliest start / latest end of this launch's CTAs (%globaltimer, ns)
-    int parts_offset;            // where in shared memory the cluster's parts arrive (bytes)
-    int cluster_reduce;          // the gridDim.y CTAs of a row group are one cluster and sum their parts through the first one's shared memory
-};
 
 struct W32 {                      // 16 consecutive bfloat16 of one weight row
     uint32_t r[8];
@@ -722,6 +678,8 @@ static int gemm_skinny_any(cudaStream_t stream, int epilogue, int norm, int use_
     p.norm_mode = norm; p.ss_in = ss_in; p.ss_parts = ss_parts;
     p.resid_inout = resid_inout; p.gain_out = gain_out; p.xn_out = (bf16*)xn_out; p.ss_out = ss_out;
     p.act = act; p.act_a = act_a; p.act_b = act_b;
+    const int taken = eg_gemm_stream_launch(stream, epilogue, norm, p);
+    if (taken >= 0) return taken;
     const int ctas = (N + row_blocks * 16 - 1) / (row_blocks * 16);
 #define EG_SKINNY(E)                                                                             \
     case E: return norm == 2 ? launch_nt<E, 2>(stream, p, ctas, k_split)                          \

@@ -682,3 +682,72 @@ def test_prompt_attention_with_either_number_of_softmax_groups(groups):
                          env=env, capture_output=True, text=True, cwd=os.path.dirname(os.path.dirname(os.path.abspath(__file__))))
     assert out.returncode == 0, out.stdout[-3000:] + out.stderr[-2000:]
     assert " passed" in out.stdout
+
+
+# -- the decode product with its weights through shared memory (gemm_stream.cu) ------------------
+
+@pytest.mark.parametrize("M", [1, 7, 16])
+@pytest.mark.parametrize("N, K", [(8, 16), (900, 896), (200, 2064), (896, 4864), (1030, 8208), (6416, 80), (19001, 208)])
+def test_gemm_stream_units_splits_and_shares(M, N, K):
+    """Less than a row block, ragged last units, K whole and cut across clusters (one of them with a short last part), and
+    matrices whose CTAs walk over shares that are no whole units."""
+    from easy_gpt.cpp_b200 import kernels
+
+    x, w, b = bf(torch.randn(M, K, generator=gen(70))), bf(torch.randn(N, K, generator=gen(71)) * 0.1), torch.randn(N, generator=gen(72))
+    want = x.float() @ w.float().t() + b
+    out = torch.full((M, N), float("nan"), device=DEV)
+    kernels.gemm_skinny(w.to(DEV), b.to(DEV), out, kernels.EPI_F32, x=x.to(DEV))
+    assert float((out.cpu() - want).abs().max()) <= 1e-5 * float(want.abs().max()) * math.sqrt(K)       # float32 accumulation
+
+
+@pytest.mark.parametrize("M, H, I, J", [(1, 896, 4864, 4864), (16, 208, 2064, 9600), (9, 1040, 304, 72)])
+def test_gemm_stream_residual_norm_then_swiglu(M, H, I, J):
+    from easy_gpt.cpp_b200 import kernels
+
+    act, w = bf(torch.randn(M, I, generator=gen(73))), bf(torch.randn(H, I, generator=gen(74)) * 0.05)
+    gate_up = bf(torch.randn(2 * J, H, generator=gen(75)) * 0.05)
+    resid, gain = torch.randn(M, H, generator=gen(76)) * 2, 1 + 0.1 * torch.randn(H, generator=gen(77))
+    delta = bf(act.float() @ w.float().t()).float()
+    r = resid.to(DEV)
+    rows, ss = kernels.gemm_skinny(w.to(DEV), None, None, kernels.EPI_RESID_NORM, x=act.to(DEV), follow=dict(residual=r, gain=gain.to(DEV)))
+    v = r.cpu()
+    assert float((v - resid - delta).abs().max()) <= 2 ** -7 * float(delta.abs().max()) + 1e-6             # the delta is rounded to bfloat16
+    assert torch.equal(rows.cpu(), bf(gain * v))
+    assert torch.allclose(ss.sum(0).cpu()[:M], (v * v).sum(1), rtol=1e-5)
+    out = torch.empty(M, J, dtype=torch.bfloat16, device=DEV)
+    kernels.gemm_skinny(gate_up.to(DEV), None, out, kernels.EPI_SWIGLU, prenormed=(rows, ss), eps=1e-5)
+    factor = 1 / torch.sqrt((v * v).mean(1, keepdim=True) + 1e-5)
+    y = rows.float().cpu() @ gate_up.float().t() * factor
+    want = y[:, 1::2] * torch.nn.functional.silu(y[:, 0::2])
+    assert float((out.float().cpu() - want).abs().max()) <= 2 ** -7 * float(want.abs().max())              # rounded to bfloat16
+
+
+@pytest.mark.parametrize("M, NH, NKV, HD, K", [(1, 14, 2, 64, 896), (16, 3, 1, 96, 1616), (5, 12, 2, 128, 1536), (3, 2, 2, 32, 64)])
+def test_gemm_stream_qkv_rope_cache(M, NH, NKV, HD, K):
+    """Pairs of row blocks per head, K whole and cut in two, a head of three pairs: against product, rotation and cache rows."""
+    from easy_gpt.cpp_b200 import kernels
+    from easy_gpt.cpp_b200.parts.rope import RotaryEncoding
+
+    ps, pages, N = 16, 9, (NH + 2 * NKV) * HD
+    w, bias = bf(torch.randn(N, K, generator=gen(80)) * 0.05), torch.randn(N, generator=gen(81)) * 0.3
+    rows, ss = bf(torch.randn(M, K, generator=gen(82))), torch.zeros(3, kernels.skinny_padded_tokens(M))
+    ss[:, :M] = torch.rand(3, M, generator=gen(83)) * K
+    positions = torch.randint(0, 5000, (M,), generator=gen(84), dtype=torch.int32)
+    slots = torch.randperm(ps * pages, generator=gen(85))[:M].to(torch.int32)
+    inv, status = RotaryEncoding.inverse_frequencies(HD, 1e6), torch.zeros(1, dtype=torch.int32, device=DEV)
+    kc = torch.zeros(pages, NKV, ps, HD, dtype=torch.bfloat16, device=DEV)
+    vc, q = torch.zeros_like(kc), torch.empty(M, NH * HD, dtype=torch.bfloat16, device=DEV)
+    kernels.gemm_skinny(w.to(DEV), bias.to(DEV), q, kernels.EPI_QKV_ROPE, prenormed=(rows.to(DEV), ss.to(DEV)), eps=1e-6,
+                        rope=dict(num_heads=NH, num_kv_heads=NKV, head_dim=HD, positions=positions.to(DEV), slot_map=slots.to(DEV), k_cache=kc,
+                                  v_cache=vc, inv_freq=inv.to(DEV), status=status))
+    assert status.item() == 0
+    full = rows.float() @ w.float().t() / torch.sqrt(ss.sum(0)[:M, None] / K + 1e-6) + bias
+    qw = plain_model.rope(full[:, :NH * HD].reshape(M, NH, HD), positions.long(), 1e6).reshape(M, -1)
+    kw = plain_model.rope(full[:, NH * HD:(NH + NKV) * HD].reshape(M, NKV, HD), positions.long(), 1e6)
+    vw = full[:, (NH + NKV) * HD:].reshape(M, NKV, HD)
+    tol = 2 ** -7 * float(full.abs().max())                                                                 # rounded to bfloat16
+    assert float((q.float().cpu() - qw).abs().max()) <= tol
+    at = (slots.long() // ps, slice(None), slots.long() % ps)
+    assert float((kc.float().cpu()[at] - kw).abs().max()) <= tol
+    assert float((vc.float().cpu()[at] - vw).abs().max()) <= tol
+    assert int((kc.float().abs().sum(dim=(1, 3)) > 0).sum()) == M
