@@ -35,7 +35,11 @@ template <class F> long long guarded(char* error, int cap, F f) {
 struct Runner {
     std::unique_ptr<Model> model;
     std::unique_ptr<StepRunner> runner;
-    std::vector<float> host_logits;
+    cudaEvent_t start = nullptr, stop = nullptr;        // around a step's launches
+    ~Runner() {
+        if (start) cudaEventDestroy(start);
+        if (stop) cudaEventDestroy(stop);
+    }
 };
 }  // namespace
 
@@ -225,12 +229,11 @@ EGE_API long long ege_runner_step(void* r, int n, const long long* rids, const l
                                   const long long* wants, float* logits, long long cap_floats, double* device_ms, char* error, int cap) {
     return guarded(error, cap, [&]() {
         Runner* run = static_cast<Runner*>(r);
-        cudaEvent_t start = nullptr, stop = nullptr;
         if (device_ms) {                        // the step's time on the device, between events on the runner's stream
-            EG_CUDA(cudaEventCreate(&start));
-            EG_CUDA(cudaEventCreate(&stop));
+            if (!run->start) EG_CUDA(cudaEventCreate(&run->start));
+            if (!run->stop) EG_CUDA(cudaEventCreate(&run->stop));
             EG_CUDA(cudaStreamSynchronize(run->runner->stream));
-            EG_CUDA(cudaEventRecord(start, run->runner->stream));
+            EG_CUDA(cudaEventRecord(run->start, run->runner->stream));
         }
         std::vector<StepEntry> entries((size_t)n);
         long long at = 0;
@@ -241,7 +244,7 @@ EGE_API long long ege_runner_step(void* r, int n, const long long* rids, const l
             at += counts[i];
         }
         const StepRunner::Result res = run->runner->run(entries, /*check=*/false, /*commit=*/true);
-        if (device_ms) EG_CUDA(cudaEventRecord(stop, run->runner->stream));
+        if (device_ms) EG_CUDA(cudaEventRecord(run->stop, run->runner->stream));
         const long long vocab = run->model->lm_head->vocab();
         if (res.rows > 0) {
             if ((long long)res.rows * vocab > cap_floats) throw std::invalid_argument("the caller's logits buffer is too small");
@@ -250,13 +253,23 @@ EGE_API long long ege_runner_step(void* r, int n, const long long* rids, const l
         run->runner->check_status();           // synchronises the stream: the logits are on the host
         if (device_ms) {
             float ms = 0.f;
-            EG_CUDA(cudaEventElapsedTime(&ms, start, stop));
+            EG_CUDA(cudaEventElapsedTime(&ms, run->start, run->stop));
             *device_ms = ms;
-            cudaEventDestroy(start);
-            cudaEventDestroy(stop);
         }
         return (long long)res.rows;
     });
+}
+// Page-locked host memory that a step's logits can be copied to at the link's rate; nullptr if there is none to be had.
+EGE_API void* ege_host_alloc(long long bytes) {
+    void* p = nullptr;
+    if (bytes <= 0 || cudaHostAlloc(&p, (size_t)bytes, cudaHostAllocDefault) != cudaSuccess) {
+        (void)cudaGetLastError();
+        return nullptr;
+    }
+    return p;
+}
+EGE_API void ege_host_free(void* p) {
+    if (p) cudaFreeHost(p);
 }
 EGE_API void ege_runner_end(void* r, long long rid) { static_cast<Runner*>(r)->runner->end(rid); }
 // what: 0 vocabulary, 1 live requests, 2 captured-step replays, 3 free pages of group `arg`, 4 pages of group `arg`, 5 pages handed

@@ -8,7 +8,10 @@ tokens in, float32 logits at the wanted places out.  The same library is what th
 """
 from __future__ import annotations
 
+import collections
 import ctypes
+import threading
+import weakref
 from ctypes import POINTER, c_char_p, c_float, c_int, c_longlong, c_void_p
 from typing import Dict, Hashable, List, Optional, Sequence
 
@@ -55,6 +58,8 @@ def library() -> ctypes.CDLL:
             "ege_runner_step": (c_longlong, [c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_longlong, c_void_p, c_char_p, c_int]),
             "ege_runner_end": (None, [c_void_p, c_longlong]),
             "ege_runner_info": (c_longlong, [c_void_p, c_int, c_int]),
+            "ege_host_alloc": (c_void_p, [c_longlong]),
+            "ege_host_free": (None, [c_void_p]),
             "ege_plan": (None, [c_int, c_void_p, c_void_p]),
         }
         for name, (restype, argtypes) in sig.items():
@@ -219,6 +224,66 @@ class NativeEngine:
         return outputs
 
 
+class _HostBlocks:
+    """Page-locked host memory for the logits that a runner hands out, taken again once the array (and every view of it) is
+    gone.  The copy from the device into fresh pageable memory was most of a decode step of several requests: 16 rows of
+    151,936 logits took 2.1 to 4 ms behind a step of 1.4 ms, into page-locked memory 0.2.  At most LIMIT bytes are held;
+    beyond that, and for arrays of less than GRAIN bytes (where the copy costs nothing), the caller uses plain memory."""
+
+    LIMIT, GRAIN = 512 << 20, 64 << 10
+
+    def __init__(self, lib):
+        self._lib, self._lock, self._closed, self._held = lib, threading.Lock(), False, 0
+        self._free = {}                                          # size -> addresses
+        self._returned = collections.deque()                     # (address, size): finalizers may run anywhere, so they take no lock
+
+    def array(self, rows: int, columns: int):
+        """An uninitialised float32 array [rows, columns], or None."""
+        size = -(-rows * columns * 4 // self.GRAIN) * self.GRAIN
+        if rows * columns * 4 < self.GRAIN:
+            return None
+        with self._lock:
+            while self._returned:
+                at, n = self._returned.popleft()
+                self._free.setdefault(n, []).append(at)
+            if self._free.get(size):
+                address = self._free[size].pop()
+            else:
+                for n, blocks in self._free.items():             # blocks of other sizes make room
+                    while blocks and self._held + size > self.LIMIT:
+                        self._lib.ege_host_free(blocks.pop())
+                        self._held -= n
+                address = self._lib.ege_host_alloc(size) if self._held + size <= self.LIMIT else None
+                if not address:
+                    return None
+                self._held += size
+        memory = (c_float * (rows * columns)).from_address(address)
+        weakref.finalize(memory, self._give_back, address, size).atexit = False
+        return np.frombuffer(memory, dtype=np.float32).reshape(rows, columns)
+
+    def _give_back(self, address: int, size: int) -> None:
+        self._returned.append((address, size))
+        if self._closed:
+            self._drop_returned()
+
+    def _drop_returned(self) -> None:
+        while True:
+            try:
+                address, _ = self._returned.popleft()
+            except IndexError:
+                return
+            self._lib.ege_host_free(address)
+
+    def close(self) -> None:
+        """Frees what is not handed out; the rest is freed as its arrays go."""
+        self._closed = True
+        self._drop_returned()
+        with self._lock:
+            for blocks in self._free.values():
+                while blocks:
+                    self._lib.ege_host_free(blocks.pop())
+
+
 class NativeStepRunner:
     """The step function alone: ``run`` takes entries (request, tokens, want) and returns float32 logits [wanted, vocab]
     as a numpy array (None if nothing is wanted)."""
@@ -233,6 +298,7 @@ class NativeStepRunner:
             raise NativeError(self._err.value.decode(errors="replace"))
         self.vocab = int(self._lib.ege_runner_info(self._h, 0, 0))
         self._device_ms = np.zeros(1, dtype=np.float64)
+        self._blocks = _HostBlocks(self._lib)
         self._handles: Dict[Hashable, int] = {}
         self._next = 1 << 40
 
@@ -240,6 +306,7 @@ class NativeStepRunner:
         h, self._h = getattr(self, "_h", None), None
         if h:
             self._lib.ege_runner_destroy(h)
+            self._blocks.close()
 
     def _handle(self, rid) -> int:
         if isinstance(rid, (int, np.integer)) and not isinstance(rid, bool) and 0 <= int(rid) < (1 << 40):
@@ -260,7 +327,9 @@ class NativeStepRunner:
         want_offsets[1:] = np.cumsum([len(w) for _, _, w in triples])
         wants = np.asarray([x for _, _, w in triples for x in w] or [0], dtype=np.int64)
         rows = int(want_offsets[n])
-        logits = np.empty((max(rows, 1), self.vocab), dtype=np.float32)
+        logits = self._blocks.array(rows, self.vocab) if rows else None
+        if logits is None:
+            logits = np.empty((max(rows, 1), self.vocab), dtype=np.float32)
         got = self._lib.ege_runner_step(self._h, n, rids.ctypes.data, counts.ctypes.data, tokens.ctypes.data, want_offsets.ctypes.data,
                                         wants.ctypes.data, logits.ctypes.data, logits.size, self._device_ms.ctypes.data, self._err, _ERR)
         if got < 0:
