@@ -751,3 +751,29 @@ def test_gemm_stream_qkv_rope_cache(M, NH, NKV, HD, K):
     assert float((kc.float().cpu()[at] - kw).abs().max()) <= tol
     assert float((vc.float().cpu()[at] - vw).abs().max()) <= tol
     assert int((kc.float().abs().sum(dim=(1, 3)) > 0).sum()) == M
+
+
+@pytest.mark.parametrize("NH, NKV, HD, ps, contexts, queries, window", [
+    (9, 1, 30, 4, [5, 290], [3, 1], None),          # rows that are no whole pieces of four; more query heads than a CTA has room for
+    (3, 3, 96, 8, [600], [2], None),                # one query head per KV head, chunks come round on four warps
+    (16, 2, 128, 16, [1055, 31], [1, 2], 900),      # eight query heads, a window that starts inside a chunk
+    (6, 2, 20, 16, [255, 256], [1, 1], None),       # the last chunk ends and begins
+    (5, 1, 200, 16, [40], [70], 33),
+])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_attention_generic_chunks_and_head_groups(NH, NKV, HD, ps, contexts, queries, window, dtype):
+    from easy_gpt.cpp_b200 import kernels
+
+    c = paged_case(13, NH, NKV, HD, ps, contexts, queries, dtype, window)
+    args = [c[k].to(DEV) for k in ("q", "kc", "vc", "table", "token_seq", "positions")]
+    status, T = torch.zeros(1, dtype=torch.int32, device=DEV), c["q"].shape[0]
+    out = torch.zeros(T, NH * HD, dtype=dtype, device=DEV)
+    kernels.attention_generic(*args, out, NH, NKV, HD, window, 1.0 / math.sqrt(HD), status)
+    assert status.item() == 0
+    # float32 sums; bfloat16: the result's rounding (values of order one)
+    assert float((out.float().cpu() - c["want"]).abs().max()) <= (2e-5 if dtype == torch.float32 else 2.5e-2)
+    # a token's result does not hang off what else is in the step
+    alone = torch.zeros(1, NH * HD, dtype=dtype, device=DEV)
+    kernels.attention_generic(args[0][T - 1:].contiguous(), *args[1:4], args[4][T - 1:].contiguous(), args[5][T - 1:].contiguous(), alone, NH, NKV, HD, window,
+                              1.0 / math.sqrt(HD), status)
+    assert torch.equal(alone[0], out[T - 1])
