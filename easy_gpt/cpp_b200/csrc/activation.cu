@@ -20,6 +20,7 @@ __global__ void swiglu_kernel(const T* __restrict__ gate_up, int ld, T* __restri
 // Four outputs per thread: one 16-byte (bfloat16) or two 16-byte (float32) loads, one vector store.
 template <typename T>
 __global__ void swiglu_vec4_kernel(const T* __restrict__ gate_up, int ld, T* __restrict__ out, int ldo, int inter) {
+    pdl_enter();
     const int t = blockIdx.x;
     const int i = (blockIdx.y * blockDim.x + threadIdx.x) * 4;
     if (i >= inter) return;
@@ -62,9 +63,9 @@ EG_API int eg_swiglu(cudaStream_t stream, int dtype, const void* gate_up, int ld
         ((uintptr_t)gate_up % 16) == 0 && ((uintptr_t)out % (4 * es)) == 0) {
         dim3 vgrid(tokens, (inter / 4 + 127) / 128);
         if (dtype == EG_BF16)
-            swiglu_vec4_kernel<bf16><<<vgrid, 128, 0, stream>>>((const bf16*)gate_up, ld, (bf16*)out, ldo, inter);
+            eg_pdl_launch(swiglu_vec4_kernel<bf16>, vgrid, 128, 0, stream, (const bf16*)gate_up, ld, (bf16*)out, ldo, inter);
         else
-            swiglu_vec4_kernel<float><<<vgrid, 128, 0, stream>>>((const float*)gate_up, ld, (float*)out, ldo, inter);
+            eg_pdl_launch(swiglu_vec4_kernel<float>, vgrid, 128, 0, stream, (const float*)gate_up, ld, (float*)out, ldo, inter);
         return eg_launch_status();
     }
     dim3 grid(tokens, (inter + 255) / 256);
@@ -166,6 +167,7 @@ namespace {
 template <bool PER_VALUE>
 __global__ void __launch_bounds__(256) sigmoid_gate_vec_kernel(bf16* __restrict__ values, long long ldv, const float* __restrict__ gate, long long ldg, int tokens, int n,
                                                                int span) {
+    pdl_enter();
     const int pieces = n / 8;
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= (long long)tokens * pieces) return;
@@ -194,8 +196,8 @@ EG_API int eg_sigmoid_gate(cudaStream_t stream, int dtype, void* values, long lo
     const unsigned blocks = (unsigned)((total + 255) / 256);
     if (dtype == EG_BF16 && n % 8 == 0 && ldv % 8 == 0 && (span == 1 || span % 8 == 0) && (uintptr_t)values % 16 == 0) {
         const unsigned vec_blocks = (unsigned)((total / 8 + 255) / 256);
-        if (span == 1) sigmoid_gate_vec_kernel<true><<<vec_blocks, 256, 0, stream>>>((bf16*)values, ldv, gate, ldg, tokens, n, span);
-        else sigmoid_gate_vec_kernel<false><<<vec_blocks, 256, 0, stream>>>((bf16*)values, ldv, gate, ldg, tokens, n, span);
+        if (span == 1) eg_pdl_launch(sigmoid_gate_vec_kernel<true>, vec_blocks, 256, 0, stream, (bf16*)values, ldv, gate, ldg, tokens, n, span);
+        else eg_pdl_launch(sigmoid_gate_vec_kernel<false>, vec_blocks, 256, 0, stream, (bf16*)values, ldv, gate, ldg, tokens, n, span);
         return eg_launch_status();
     }
     if (dtype == EG_BF16) sigmoid_gate_kernel<bf16><<<blocks, 256, 0, stream>>>((bf16*)values, ldv, gate, ldg, tokens, n, span);

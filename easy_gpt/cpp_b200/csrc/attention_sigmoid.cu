@@ -78,6 +78,7 @@ __global__ void __launch_bounds__(256) sigmoid_prepare_kernel(const float* __res
                                                               T* __restrict__ k_cache, T* __restrict__ v_cache, int row_stride, long long head_stride,
                                                               int page_size, long long page_stride, long long pool_slots, T* __restrict__ q_out, int nq, int nk,
                                                               int nv, int dk, int dv, int* status) {
+    pdl_enter();
     __shared__ float scratch[32];
     const int t = blockIdx.x;
     const float* row = proj + (size_t)t * ld;
@@ -428,6 +429,7 @@ __host__ __device__ inline int range_keys(int keys, int splits) {
 
 template <int NT>
 __global__ void __launch_bounds__(SPLIT_WARPS * 32) sigmoid_split_kernel(const MmaParams p) {
+    pdl_enter();
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ int last_here;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -589,7 +591,7 @@ EG_API int eg_sigmoid_attention_prepare(cudaStream_t stream, int dtype, const fl
                       (uintptr_t)proj % 16 == 0 && (uintptr_t)bias % 16 == 0 && (uintptr_t)q_gain % 16 == 0 && (uintptr_t)k_gain % 16 == 0 &&
                       (uintptr_t)k_cache % 16 == 0 && (uintptr_t)v_cache % (dtype == EG_BF16 ? 8 : 16) == 0 && (uintptr_t)q_out % 16 == 0;
 #define EG_PREPARE(T, VEC)                                                                                                                                    \
-    sigmoid_prepare_kernel<T, VEC><<<tokens, 256, 0, stream>>>(proj, ld, bias, q_gain, k_gain, eps, temp_coef, temp_every, positions, slot_map, (T*)k_cache,   \
+    eg_pdl_launch(sigmoid_prepare_kernel<T, VEC>, tokens, 256, 0, stream, proj, ld, bias, q_gain, k_gain, eps, temp_coef, temp_every, positions, slot_map, (T*)k_cache,   \
                                                                (T*)v_cache, row_stride, head_stride, page_size, page_stride, pool_slots, (T*)q_out, nq, nk,    \
                                                                nv, dk, dv, status)
     if (dtype == EG_BF16) {
@@ -731,7 +733,7 @@ EG_API int eg_sigmoid_attention_split(cudaStream_t stream, const void* q, const 
     {                                                                                \
         const int rc = allow_smem(sigmoid_split_kernel<NT>, smem);                   \
         if (rc) return rc;                                                           \
-        sigmoid_split_kernel<NT><<<grid, SPLIT_WARPS * 32, smem, stream>>>(p);       \
+        eg_pdl_launch(sigmoid_split_kernel<NT>, grid, SPLIT_WARPS * 32, smem, stream, p);       \
     }
     const int nt = pad16(dv) / 8;
     if (nt <= 4) EG_SPLIT(4)

@@ -28,6 +28,7 @@ __global__ void __launch_bounds__(128) sink_prepare_kernel(const float* __restri
                                                            T* __restrict__ v_cache, int row_stride, long long head_stride, int page_size,
                                                            long long page_stride, long long pool_slots, T* __restrict__ q_out, int tokens, int heads,
                                                            int kv_heads, int dk, int dv, float unit_eps, int* status) {
+    pdl_enter();
     const int lane = threadIdx.x & 31;
     const long long w = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (w >= (long long)tokens * (heads + kv_heads)) return;
@@ -165,10 +166,10 @@ EG_API int eg_sink_attention_prepare(cudaStream_t stream, int dtype, const float
     const long long warps = (long long)tokens * (heads + kv_heads);
     const unsigned blocks = (unsigned)((warps + 3) / 4);
     if (dtype == EG_BF16)
-        sink_prepare_kernel<bf16><<<blocks, 128, 0, stream>>>(proj, ld, (const float2*)table, rot_dims / 2, magnitude, slot_map, (bf16*)k_cache, (bf16*)v_cache,
+        eg_pdl_launch(sink_prepare_kernel<bf16>, blocks, 128, 0, stream, proj, ld, (const float2*)table, rot_dims / 2, magnitude, slot_map, (bf16*)k_cache, (bf16*)v_cache,
                                                               row_stride, head_stride, page_size, page_stride, pool_slots, (bf16*)q_out, tokens, heads, kv_heads, dk, dv, unit_eps, status);
     else
-        sink_prepare_kernel<float><<<blocks, 128, 0, stream>>>(proj, ld, (const float2*)table, rot_dims / 2, magnitude, slot_map, (float*)k_cache, (float*)v_cache,
+        eg_pdl_launch(sink_prepare_kernel<float>, blocks, 128, 0, stream, proj, ld, (const float2*)table, rot_dims / 2, magnitude, slot_map, (float*)k_cache, (float*)v_cache,
                                                                row_stride, head_stride, page_size, page_stride, pool_slots, (float*)q_out, tokens, heads, kv_heads, dk, dv, unit_eps, status);
     return eg_launch_status();
 }

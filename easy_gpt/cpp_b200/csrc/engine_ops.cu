@@ -76,6 +76,7 @@ __global__ void add_bias_rows_kernel(float* __restrict__ x, long long ld, const 
 }
 template <typename TD>
 __global__ void convert_columns_kernel(const float* __restrict__ src, long long lds, TD* __restrict__ dst, long long ldd, int rows, int cols, int padded) {
+    pdl_enter();
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= (long long)rows * padded) return;
     const int c = (int)(i % padded);
@@ -99,7 +100,7 @@ EG_API int eg_convert_columns(cudaStream_t stream, const float* src, long long l
     if (n <= 0) return 0;
     if (padded < cols) return (int)cudaErrorInvalidValue;
     const unsigned blocks = (unsigned)((n + 255) / 256);
-    if (dst_dtype == EG_BF16) convert_columns_kernel<bf16><<<blocks, 256, 0, stream>>>(src, lds, (bf16*)dst, ldd, rows, cols, padded);
-    else convert_columns_kernel<float><<<blocks, 256, 0, stream>>>(src, lds, (float*)dst, ldd, rows, cols, padded);
+    if (dst_dtype == EG_BF16) eg_pdl_launch(convert_columns_kernel<bf16>, blocks, 256, 0, stream, src, lds, (bf16*)dst, ldd, rows, cols, padded);
+    else eg_pdl_launch(convert_columns_kernel<float>, blocks, 256, 0, stream, src, lds, (float*)dst, ldd, rows, cols, padded);
     return eg_launch_status();
 }

@@ -201,6 +201,7 @@ __device__ __forceinline__ void make_records(const DeltaParams& p, int DS, int t
 // a group of p.lanes lanes (a power of two up to 32) per (block of tokens, head)
 template <int CH, bool WIDE>
 __global__ void __launch_bounds__(128) general_delta_records_kernel(const DeltaParams p, int DS, int num_seqs) {
+    pdl_enter();
     const int group = p.lanes, lane = threadIdx.x % group;
     const long long i = ((long long)blockIdx.x * blockDim.x + threadIdx.x) / group;
     // neighbouring groups take neighbouring heads of a block: the projection's rows are read in order
@@ -236,6 +237,7 @@ __device__ __forceinline__ void norm_and_gate(const DeltaParams& p, const float*
 // behind a recurrence whose blocks held slices of a head: `lanes` lanes per (token, head), four channels a lane and pass (WIDE)
 template <typename TO, bool WIDE>
 __global__ void __launch_bounds__(256) general_delta_output_kernel(const DeltaParams p) {
+    pdl_enter();
     if (!WIDE) {
         const long long i = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
         if (i >= (long long)p.tokens * p.heads) return;
@@ -274,6 +276,7 @@ __global__ void __launch_bounds__(256) general_delta_output_kernel(const DeltaPa
 // INLINE: the block makes its entry's records itself (entries of up to p.tile tokens)
 template <typename TO, int R, int P, int COLS, bool INLINE>
 __global__ void __launch_bounds__(INLINE ? 512 : 256, 1) general_delta_kernel(const DeltaParams p) {
+    pdl_enter();
     extern __shared__ __align__(128) float smem[];
     __shared__ __align__(8) uint64_t full[STAGES];
     __shared__ int abort_flag;
@@ -595,16 +598,18 @@ int launch_general_delta(cudaStream_t stream, DeltaParams p, int slices, int num
         constexpr int CH = DS <= 128 ? 1 : 2;
         p.lanes = DS / 4 / CH;
         const unsigned blocks = (unsigned)(((long long)(p.tokens / BLOCK + num_seqs) * p.heads * p.lanes + 127) / 128);
-        if (wide) general_delta_records_kernel<CH, true><<<blocks, 128, 0, stream>>>(p, DS, num_seqs);
-        else general_delta_records_kernel<CH, false><<<blocks, 128, 0, stream>>>(p, DS, num_seqs);
+        if (wide) eg_pdl_launch(general_delta_records_kernel<CH, true>, blocks, 128, 0, stream, p, DS, num_seqs);
+        else eg_pdl_launch(general_delta_records_kernel<CH, false>, blocks, 128, 0, stream, p, DS, num_seqs);
     }
-    kernel<<<dim3(p.heads, num_seqs, slices), cols / COLS * P, smem, stream>>>(p);
+    // (prompts: its blocks, about one an SM, find their SMs evenly only when the kernel in front has left them; placed early a
+    // prompt of 2,047 tokens through six layers took 3.48 ms, placed after it 3.03)
+    eg_pdl_launch_if(p.tokens <= 4 * num_seqs, kernel, dim3(p.heads, num_seqs, slices), cols / COLS * P, smem, stream, p);
     if (p.o_raw) {
         if (wide) {
             p.lanes = power_of_two_lanes((p.dim + 3) / 4);
-            general_delta_output_kernel<TO, true><<<(unsigned)(((long long)p.tokens * p.heads * p.lanes + 255) / 256), 256, 0, stream>>>(p);
+            eg_pdl_launch(general_delta_output_kernel<TO, true>, (unsigned)(((long long)p.tokens * p.heads * p.lanes + 255) / 256), 256, 0, stream, p);
         } else {
-            general_delta_output_kernel<TO, false><<<(unsigned)(((long long)p.tokens * p.heads + 7) / 8), 256, 0, stream>>>(p);
+            eg_pdl_launch(general_delta_output_kernel<TO, false>, (unsigned)(((long long)p.tokens * p.heads + 7) / 8), 256, 0, stream, p);
         }
     }
     return eg_launch_status();
@@ -625,6 +630,7 @@ int dispatch_general_delta(cudaStream_t stream, const DeltaParams& p, int slices
 
 template <typename T>
 __global__ void tanh_columns_kernel(const float* __restrict__ src, long long lds, T* __restrict__ dst, long long ldd, int rows, int cols, int padded) {
+    pdl_enter();
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= (long long)rows * padded) return;
     const int t = (int)(i / padded), c = (int)(i % padded);
@@ -699,7 +705,7 @@ EG_API int eg_general_delta(cudaStream_t stream, const float* proj, long long ld
 EG_API int eg_tanh_columns(cudaStream_t stream, const float* src, long long lds, void* dst, int dst_dtype, long long ldd, int rows, int cols, int padded) {
     if (rows <= 0 || padded <= 0) return 0;
     const unsigned blocks = (unsigned)(((long long)rows * padded + 255) / 256);
-    if (dst_dtype == EG_BF16) tanh_columns_kernel<bf16><<<blocks, 256, 0, stream>>>(src, lds, (bf16*)dst, ldd, rows, cols, padded);
-    else tanh_columns_kernel<float><<<blocks, 256, 0, stream>>>(src, lds, (float*)dst, ldd, rows, cols, padded);
+    if (dst_dtype == EG_BF16) eg_pdl_launch(tanh_columns_kernel<bf16>, blocks, 256, 0, stream, src, lds, (bf16*)dst, ldd, rows, cols, padded);
+    else eg_pdl_launch(tanh_columns_kernel<float>, blocks, 256, 0, stream, src, lds, (float*)dst, ldd, rows, cols, padded);
     return eg_launch_status();
 }

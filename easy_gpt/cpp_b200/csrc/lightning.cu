@@ -59,6 +59,7 @@ struct LightningParams {
 // ---- short entries -------------------------------------------------------------------------------------------------------------
 template <int R, int P>
 __global__ void __launch_bounds__(512, 1) lightning_short_kernel(const LightningParams p) {
+    pdl_enter();
     extern __shared__ __align__(16) float smem[];
     constexpr int DS = R * P;
     const int cols = p.cols, dk = p.dk, dv = p.dv;
@@ -490,6 +491,7 @@ __global__ void __launch_bounds__(256, 2) lightning_out_mma_kernel(const Lightni
 template <typename TO, int VEC>
 __global__ void __launch_bounds__(256) lightning_output_kernel(const float* __restrict__ o_raw, const float* __restrict__ proj, long long ldp, int g_col,
                                                                const float* __restrict__ gain, TO* __restrict__ y, long long ldy, int n, float eps) {
+    pdl_enter();
     __shared__ float scratch[32];
     const int t = blockIdx.x;
     const float* o = o_raw + (size_t)t * n;
@@ -531,7 +533,7 @@ int launch_short(cudaStream_t stream, LightningParams p, int slices) {
     slices = (p.dv + cols - 1) / cols;
     p.cols = cols;
     const size_t smem = (size_t)TILE * (2 * R * P + cols) * sizeof(float);
-    lightning_short_kernel<R, P><<<dim3(p.heads, p.num_seqs, slices), cols * P, smem, stream>>>(p);
+    eg_pdl_launch(lightning_short_kernel<R, P>, dim3(p.heads, p.num_seqs, slices), cols * P, smem, stream, p);
     return 0;
 }
 }  // namespace
@@ -595,7 +597,7 @@ EG_API int eg_lightning(cudaStream_t stream, const float* proj, long long ldp, i
     const int n = heads * dv;
     const bool wide = n % 4 == 0 && ldp % 4 == 0 && g_col % 4 == 0 && ldy % 4 == 0 && (uintptr_t)proj % 16 == 0 && (uintptr_t)o_raw % 16 == 0 &&
                       (uintptr_t)gain % 16 == 0 && (uintptr_t)y % 16 == 0;
-#define EG_OUTPUT(TO, VEC) lightning_output_kernel<TO, VEC><<<tokens, 256, 0, stream>>>(o_raw, proj, ldp, g_col, gain, (TO*)y, ldy, n, eps)
+#define EG_OUTPUT(TO, VEC) eg_pdl_launch(lightning_output_kernel<TO, VEC>, tokens, 256, 0, stream, o_raw, proj, ldp, g_col, gain, (TO*)y, ldy, n, eps)
     if (y_dtype == EG_BF16) {
         if (wide) EG_OUTPUT(bf16, 4);
         else EG_OUTPUT(bf16, 1);

@@ -55,6 +55,7 @@ template <typename TD, typename TO, int VPL, bool GROUPED>
 __global__ void __launch_bounds__(256) add_rmsnorm_warp_kernel(float* __restrict__ residual, const TD* __restrict__ delta,
                                                                const int* __restrict__ rows, const float* __restrict__ gain,
                                                                TO* __restrict__ out, int num_rows, int hidden, float eps, int groups) {
+    pdl_enter();
     const int lane = threadIdx.x & 31;
     const int r = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (r >= num_rows) return;
@@ -134,7 +135,7 @@ static void launch_warp_norm(cudaStream_t stream, float* residual, const void* d
     // block, 1.58 with one)
     const int warps = num_rows >= 2048 ? 8 : num_rows >= 512 ? 2 : 1, blocks = (num_rows + warps - 1) / warps;
 #define EG_WARP_NORM(V) \
-    add_rmsnorm_warp_kernel<TD, TO, V, GROUPED><<<blocks, warps * 32, 0, stream>>>(residual, (const TD*)delta, rows, gain, (TO*)out, num_rows, hidden, eps, groups)
+    eg_pdl_launch(add_rmsnorm_warp_kernel<TD, TO, V, GROUPED>, blocks, warps * 32, 0, stream, residual, (const TD*)delta, rows, gain, (TO*)out, num_rows, hidden, eps, groups)
     if (GROUPED && vpl <= 1) EG_WARP_NORM(1);
     else if (vpl <= 4) EG_WARP_NORM(4);
     else if (vpl <= 8) EG_WARP_NORM(8);

@@ -113,6 +113,7 @@ __global__ void __launch_bounds__(256) rope_cache_vec_kernel(T* __restrict__ qkv
                                                              const int* __restrict__ slot_map, T* __restrict__ k_cache, T* __restrict__ v_cache,
                                                              int tokens, int num_heads, int num_kv_heads, int head_dim, int page_size,
                                                              long long page_stride, long long head_stride, long long pool_slots, int* status) {
+    pdl_enter();
     constexpr int VEC = 16 / sizeof(T);                              // elements of a 16-byte access
     const int half = head_dim / 2, pieces = half / VEC;              // pieces of a head's first half
     const int rot_heads = num_heads + num_kv_heads;
@@ -207,11 +208,11 @@ EG_API int eg_rope_cache_vec(cudaStream_t stream, int dtype, void* qkv, int ld, 
     const int threads = 256;
     const int blocks = (int)((work + threads - 1) / threads < (1 << 20) ? (work + threads - 1) / threads : (1 << 20));
     if (dtype == EG_BF16)
-        rope_cache_vec_kernel<bf16><<<blocks, threads, 0, stream>>>((bf16*)qkv, ld, (const float2*)table, slot_map, (bf16*)k_cache, (bf16*)v_cache,
+        eg_pdl_launch(rope_cache_vec_kernel<bf16>, blocks, threads, 0, stream, (bf16*)qkv, ld, (const float2*)table, slot_map, (bf16*)k_cache, (bf16*)v_cache,
                                                                     tokens, num_heads, num_kv_heads, head_dim, page_size, page_stride,
                                                                     head_stride, pool_slots, status);
     else
-        rope_cache_vec_kernel<float><<<blocks, threads, 0, stream>>>((float*)qkv, ld, (const float2*)table, slot_map, (float*)k_cache,
+        eg_pdl_launch(rope_cache_vec_kernel<float>, blocks, threads, 0, stream, (float*)qkv, ld, (const float2*)table, slot_map, (float*)k_cache,
                                                                      (float*)v_cache, tokens, num_heads, num_kv_heads, head_dim, page_size,
                                                                      page_stride, head_stride, pool_slots, status);
     return eg_launch_status();

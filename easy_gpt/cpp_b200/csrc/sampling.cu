@@ -54,6 +54,7 @@ __device__ __forceinline__ ArgMax block_argmax(ArgMax a, ArgMax* scratch) {
 __global__ void __launch_bounds__(ARGMAX_THREADS)
 argmax_kernel(const float* __restrict__ logits, long long ld, int vocab, int* __restrict__ out,
               float* __restrict__ part_val, int* __restrict__ part_idx, int* __restrict__ counters) {
+    pdl_enter();
     __shared__ ArgMax scratch[32];
     __shared__ int is_last;
     const int r = blockIdx.x, nb = gridDim.y;
@@ -132,7 +133,7 @@ EG_API int eg_argmax(cudaStream_t stream, const float* logits, long long ld, int
     if (rows <= 0) return 0;
     if (blocks_per_row < 1 || blocks_per_row > ARGMAX_THREADS || (blocks_per_row > 1 && (!part_val || !part_idx || !counters)))
         return (int)cudaErrorInvalidValue;
-    argmax_kernel<<<dim3(rows, blocks_per_row), ARGMAX_THREADS, 0, stream>>>(logits, ld, vocab, out, part_val, part_idx, counters);
+    eg_pdl_launch(argmax_kernel, dim3(rows, blocks_per_row), ARGMAX_THREADS, 0, stream, logits, ld, vocab, out, part_val, part_idx, counters);
     return eg_launch_status();
 }
 

@@ -43,6 +43,9 @@ template <typename TO>
 __global__ void rmsnorm_shift_kernel(const float* __restrict__ stream, const float* __restrict__ gain, float eps, const float* __restrict__ mu,
                                      float* __restrict__ state, long long slot_floats, const int* __restrict__ token_seq,
                                      const int* __restrict__ seq_starts, const int* __restrict__ seq_slots, TO* __restrict__ out, int hidden) {
+    prefetch_weights(gain, hidden);
+    prefetch_weights(mu, hidden);
+    pdl_enter();
     __shared__ float scratch[32];
     const int t = blockIdx.x, seq = token_seq[t], start = seq_starts[seq];
     const bool first = t == start;
@@ -102,6 +105,8 @@ __device__ __forceinline__ float squares(float4 v) { return v.x * v.x + v.y * v.
 template <typename TD, int VPL>
 __global__ void __launch_bounds__(256) rmsnorm_add_warp_kernel(float* __restrict__ stream, const TD* __restrict__ y, long long ldy,
                                                                const float* __restrict__ gain, float eps, int tokens, int hidden) {
+    prefetch_weights(gain, hidden);
+    pdl_enter();
     const int lane = threadIdx.x & 31;
     const int t = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (t >= tokens) return;
@@ -136,6 +141,8 @@ template <typename TD, typename TO, int VPL>
 __global__ void __launch_bounds__(256) rmsnorm_add_rows_warp_kernel(float* __restrict__ stream, const TD* __restrict__ y, long long ldy,
                                                                     const float* __restrict__ bias, const float* __restrict__ gain, float eps,
                                                                     TO* __restrict__ out, int tokens, int hidden) {
+    prefetch_weights(gain, hidden);
+    pdl_enter();
     const int lane = threadIdx.x & 31;
     const int t = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (t >= tokens) return;
@@ -180,6 +187,9 @@ template <typename TD, typename TO, int VPL>
 __global__ void __launch_bounds__(256) rmsnorm_add_norm_warp_kernel(float* __restrict__ stream, const TD* __restrict__ y, long long ldy,
                                                                     const float* __restrict__ gain, float eps, const float* __restrict__ gain2,
                                                                     float eps2, TO* __restrict__ out, int tokens, int hidden) {
+    prefetch_weights(gain, hidden);
+    prefetch_weights(gain2, hidden);
+    pdl_enter();
     const int lane = threadIdx.x & 31;
     const int t = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (t >= tokens) return;
@@ -224,6 +234,9 @@ __global__ void __launch_bounds__(256) rmsnorm_shift_warp_kernel(const float* __
                                                                  const float* __restrict__ mu, float* __restrict__ state, long long slot_floats,
                                                                  const int* __restrict__ token_seq, const int* __restrict__ seq_starts,
                                                                  const int* __restrict__ seq_slots, TO* __restrict__ out, int tokens, int hidden) {
+    prefetch_weights(gain, hidden);
+    prefetch_weights(mu, hidden);
+    pdl_enter();
     __shared__ float inv_of_warp[8];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int t = blockIdx.x * (blockDim.x >> 5) + warp;
@@ -281,6 +294,9 @@ __global__ void __launch_bounds__(256) rmsnorm_shift_warp_kernel(const float* __
 template <int VPL>
 __global__ void __launch_bounds__(256) rmsnorm_pair_warp_kernel(const float* a, const float* __restrict__ b, const float* __restrict__ gain_a,
                                                                 const float* __restrict__ gain_b, float eps, float factor, float* out, int tokens, int hidden) {
+    prefetch_weights(gain_a, hidden);
+    prefetch_weights(gain_b, hidden);
+    pdl_enter();
     const int lane = threadIdx.x & 31, t = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (t >= tokens) return;
     const int quads = hidden / 4;
@@ -388,7 +404,7 @@ EG_API int eg_rmsnorm_shift(cudaStream_t stream, const float* residual, const fl
         const int nt = 128, blocks = (tokens + 3) / 4;
         const int vpl = (hidden / 4 + 31) / 32;
 #define EG_SHIFT_WARP(TO, V) \
-    rmsnorm_shift_warp_kernel<TO, V><<<blocks, nt, 0, stream>>>(residual, gain, eps, mu, state, slot_floats, token_seq, seq_starts, seq_slots, (TO*)out, tokens, hidden)
+    eg_pdl_launch(rmsnorm_shift_warp_kernel<TO, V>, blocks, nt, 0, stream, residual, gain, eps, mu, state, slot_floats, token_seq, seq_starts, seq_slots, (TO*)out, tokens, hidden)
         if (out_dtype == EG_BF16) {
             if (vpl <= 4) EG_SHIFT_WARP(bf16, 4);
             else if (vpl <= 8) EG_SHIFT_WARP(bf16, 8);
@@ -403,10 +419,10 @@ EG_API int eg_rmsnorm_shift(cudaStream_t stream, const float* residual, const fl
     }
     const int threads = row_threads(hidden);
     if (out_dtype == EG_BF16)
-        rmsnorm_shift_kernel<bf16><<<tokens, threads, 0, stream>>>(residual, gain, eps, mu, state, slot_floats, token_seq, seq_starts, seq_slots, (bf16*)out,
+        eg_pdl_launch(rmsnorm_shift_kernel<bf16>, tokens, threads, 0, stream, residual, gain, eps, mu, state, slot_floats, token_seq, seq_starts, seq_slots, (bf16*)out,
                                                                    hidden);
     else
-        rmsnorm_shift_kernel<float><<<tokens, threads, 0, stream>>>(residual, gain, eps, mu, state, slot_floats, token_seq, seq_starts, seq_slots, (float*)out,
+        eg_pdl_launch(rmsnorm_shift_kernel<float>, tokens, threads, 0, stream, residual, gain, eps, mu, state, slot_floats, token_seq, seq_starts, seq_slots, (float*)out,
                                                                     hidden);
     return eg_launch_status();
 }
@@ -419,7 +435,7 @@ EG_API int eg_rmsnorm_add(cudaStream_t stream, float* residual, const void* y, i
         int blocks, nt;
         warp_rows_launch(tokens, &blocks, &nt);
         const int vpl = (hidden / 4 + 31) / 32;
-#define EG_ADD_WARP(TD, V) rmsnorm_add_warp_kernel<TD, V><<<blocks, nt, 0, stream>>>(residual, (const TD*)y, ldy, gain, eps, tokens, hidden)
+#define EG_ADD_WARP(TD, V) eg_pdl_launch(rmsnorm_add_warp_kernel<TD, V>, blocks, nt, 0, stream, residual, (const TD*)y, ldy, gain, eps, tokens, hidden)
         if (y_dtype == EG_BF16) {
             if (vpl <= 4) EG_ADD_WARP(bf16, 4);
             else if (vpl <= 8) EG_ADD_WARP(bf16, 8);
@@ -451,7 +467,7 @@ EG_API int eg_rmsnorm_add_norm(cudaStream_t stream, float* residual, const void*
     warp_rows_launch(tokens, &blocks, &nt);
     const int vpl = (hidden / 4 + 31) / 32;
 #define EG_ADD_NORM(TD, TO, V) \
-    rmsnorm_add_norm_warp_kernel<TD, TO, V><<<blocks, nt, 0, stream>>>(residual, (const TD*)y, ldy, gain, eps, gain2, eps2, (TO*)out, tokens, hidden)
+    eg_pdl_launch(rmsnorm_add_norm_warp_kernel<TD, TO, V>, blocks, nt, 0, stream, residual, (const TD*)y, ldy, gain, eps, gain2, eps2, (TO*)out, tokens, hidden)
 #define EG_ADD_NORM_V(TD, TO)               \
     if (vpl <= 4) EG_ADD_NORM(TD, TO, 4);   \
     else if (vpl <= 8) EG_ADD_NORM(TD, TO, 8); \
@@ -478,7 +494,7 @@ EG_API int eg_rmsnorm_add_rows(cudaStream_t stream, float* residual, const void*
     warp_rows_launch(tokens, &blocks, &nt);
     const int vpl = (hidden / 4 + 31) / 32;
 #define EG_ADD_ROWS(TD, TO, V) \
-    rmsnorm_add_rows_warp_kernel<TD, TO, V><<<blocks, nt, 0, stream>>>(residual, (const TD*)y, ldy, bias, gain, eps, (TO*)out, tokens, hidden)
+    eg_pdl_launch(rmsnorm_add_rows_warp_kernel<TD, TO, V>, blocks, nt, 0, stream, residual, (const TD*)y, ldy, bias, gain, eps, (TO*)out, tokens, hidden)
 #define EG_ADD_ROWS_V(TD, TO)                  \
     if (vpl <= 4) EG_ADD_ROWS(TD, TO, 4);      \
     else if (vpl <= 8) EG_ADD_ROWS(TD, TO, 8); \
@@ -529,7 +545,7 @@ EG_API int eg_rmsnorm_pair(cudaStream_t stream, const float* a, const float* b, 
         int blocks, threads;
         warp_rows_launch(tokens, &blocks, &threads);
         const int vpl = (hidden / 4 + 31) / 32;
-#define EG_PAIR(V) rmsnorm_pair_warp_kernel<V><<<blocks, threads, 0, stream>>>(a, b, gain_a, gain_b, eps, factor, out, tokens, hidden)
+#define EG_PAIR(V) eg_pdl_launch(rmsnorm_pair_warp_kernel<V>, blocks, threads, 0, stream, a, b, gain_a, gain_b, eps, factor, out, tokens, hidden)
         if (vpl <= 4) EG_PAIR(4);
         else if (vpl <= 8) EG_PAIR(8);
         else EG_PAIR(16);

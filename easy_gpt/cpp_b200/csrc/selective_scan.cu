@@ -56,6 +56,7 @@ __global__ void conv_silu_vec4_kernel(const float* __restrict__ x, long long ldx
                                       const float* __restrict__ state, long long slot_floats, const int* __restrict__ token_seq,
                                       const int* __restrict__ seq_starts, const int* __restrict__ seq_slots, float* __restrict__ u, long long ldu,
                                       int tokens, int channels, int taps) {
+    pdl_enter();
     const int quads = channels / 4;
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= (long long)tokens * quads) return;
@@ -81,6 +82,7 @@ __global__ void conv_silu_vec4_kernel(const float* __restrict__ x, long long ldx
 template <typename T>
 __global__ void conv_state_kernel(const T* __restrict__ x, long long ldx, float* __restrict__ state, long long slot_floats,
                                   const int* __restrict__ seq_starts, const int* __restrict__ seq_slots, int num_seqs, int channels, int taps) {
+    pdl_enter();
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= (long long)num_seqs * channels) return;
     const int seq = (int)(i / channels), c = (int)(i % channels);
@@ -262,7 +264,7 @@ EG_API int eg_conv_silu(cudaStream_t stream, int dtype, const void* x, long long
     if (taps < 1) return (int)cudaErrorInvalidValue;
     if (dtype == EG_F32 && channels % 4 == 0 && ldx % 4 == 0 && ldu % 4 == 0 && slot_floats % 4 == 0 && (uintptr_t)x % 16 == 0 && (uintptr_t)u % 16 == 0 &&
         (uintptr_t)state % 16 == 0) {
-        conv_silu_vec4_kernel<<<(unsigned)((n / 4 + 255) / 256), 256, 0, stream>>>((const float*)x, ldx, conv_w, conv_b, state, slot_floats, token_seq,
+        eg_pdl_launch(conv_silu_vec4_kernel, (unsigned)((n / 4 + 255) / 256), 256, 0, stream, (const float*)x, ldx, conv_w, conv_b, state, slot_floats, token_seq,
                                                                                  seq_starts, seq_slots, (float*)u, ldu, tokens, channels, taps);
         return eg_launch_status();
     }
@@ -282,8 +284,8 @@ EG_API int eg_conv_state(cudaStream_t stream, int dtype, const void* x, long lon
     const long long n = (long long)num_seqs * channels;
     if (n <= 0 || taps <= 1) return 0;
     const unsigned blocks = (unsigned)((n + 255) / 256);
-    if (dtype == EG_BF16) conv_state_kernel<bf16><<<blocks, 256, 0, stream>>>((const bf16*)x, ldx, state, slot_floats, seq_starts, seq_slots, num_seqs, channels, taps);
-    else conv_state_kernel<float><<<blocks, 256, 0, stream>>>((const float*)x, ldx, state, slot_floats, seq_starts, seq_slots, num_seqs, channels, taps);
+    if (dtype == EG_BF16) eg_pdl_launch(conv_state_kernel<bf16>, blocks, 256, 0, stream, (const bf16*)x, ldx, state, slot_floats, seq_starts, seq_slots, num_seqs, channels, taps);
+    else eg_pdl_launch(conv_state_kernel<float>, blocks, 256, 0, stream, (const float*)x, ldx, state, slot_floats, seq_starts, seq_slots, num_seqs, channels, taps);
     return eg_launch_status();
 }
 
