@@ -102,10 +102,15 @@ __device__ __forceinline__ void store4(bf16* p, int q, float4 v) {
 }
 __device__ __forceinline__ float squares(float4 v) { return v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w; }
 
-template <typename TD, int VPL>
-__global__ void __launch_bounds__(256) rmsnorm_add_warp_kernel(float* __restrict__ stream, const TD* __restrict__ y, long long ldy,
-                                                               const float* __restrict__ gain, float eps, int tokens, int hidden) {
-    prefetch_weights(gain, hidden);
+// FEW: launches of few rows (a warp a block) keep the gain in registers too, read in front of the dependency wait
+template <typename TD, int VPL, bool FEW>
+__global__ void __launch_bounds__(FEW ? 32 : 256) rmsnorm_add_warp_kernel(float* __restrict__ stream, const TD* __restrict__ y, long long ldy,
+                                                                          const float* __restrict__ gain, float eps, int tokens, int hidden) {
+    float4 ahead[FEW ? VPL : 1];
+    if (FEW)
+#pragma unroll
+        for (int i = 0; i < VPL; ++i)
+            if (i * 32 + (int)threadIdx.x < hidden / 4) ahead[i] = load4(gain, i * 32 + threadIdx.x);
     pdl_enter();
     const int lane = threadIdx.x & 31;
     const int t = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
@@ -129,7 +134,7 @@ __global__ void __launch_bounds__(256) rmsnorm_add_warp_kernel(float* __restrict
     for (int i = 0; i < VPL; ++i) {
         const int q = i * 32 + lane;
         if (q >= quads) continue;
-        const float4 g = load4(gain, q);
+        const float4 g = FEW ? ahead[FEW ? i : 0] : load4(gain, q);
         store4(x, q, make_float4(r[i].x + g.x * (v[i].x * inv), r[i].y + g.y * (v[i].y * inv), r[i].z + g.z * (v[i].z * inv), r[i].w + g.w * (v[i].w * inv)));
     }
 }
@@ -226,6 +231,72 @@ __global__ void __launch_bounds__(256) rmsnorm_add_norm_warp_kernel(float* __res
         if (q >= quads) continue;
         const float4 g = load4(gain2, q);
         store4(out + (size_t)t * hidden, q, make_float4(g.x * (r[i].x * inv2), g.y * (r[i].y * inv2), g.z * (r[i].z * inv2), g.w * (r[i].w * inv2)));
+    }
+}
+
+// Few rows: a block per row, everything in registers and asked for at once (the weights in front of the dependency wait), both
+// rows' squares in one round through shared memory.  VPT float4 a thread.  (Measured on B200, 8 rows of 2,048 inside a decode
+// step of six such layers: two passes over both rows with a round each, and the norm-and-add behind a branch reading its gain
+// last, took 462 us a step; with this kernel and the gain ahead 423.)
+template <typename TO, int VPT>
+__global__ void __launch_bounds__(256) rmsnorm_shift_row_kernel(const float* __restrict__ stream, const float* __restrict__ gain, float eps,
+                                                                const float* __restrict__ mu, float* __restrict__ state, long long slot_floats,
+                                                                const int* __restrict__ token_seq, const int* __restrict__ seq_starts,
+                                                                const int* __restrict__ seq_slots, TO* __restrict__ out, int hidden) {
+    __shared__ float2 of_warp[8];
+    const int quads = hidden / 4, t = blockIdx.x;
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    float4 g[VPT], w[VPT], v[VPT], o[VPT], p[VPT];
+#pragma unroll
+    for (int i = 0; i < VPT; ++i) {
+        const int q = i * 256 + threadIdx.x;
+        g[i] = q < quads ? load4(gain, q) : zero;
+        w[i] = q < quads ? load4(mu, q) : zero;
+    }
+    // (the batch's tables were there before the step began)
+    const int seq = token_seq[t];
+    const bool first = t == seq_starts[seq];
+    const int behind = seq_starts[seq + 1] - 1;
+    float* slot = state + (size_t)seq_slots[seq] * slot_floats;
+    pdl_enter();
+    const float* x = stream + (size_t)t * hidden;
+    // the row in front: the stream's row t-1 normed again here, or the slot's row; the first token's block also norms the
+    // entry's last row for the slot
+    const float* other = stream + (size_t)(first ? behind : t - 1) * hidden;
+    float2 ss = make_float2(0.f, 0.f);
+#pragma unroll
+    for (int i = 0; i < VPT; ++i) {
+        const int q = i * 256 + threadIdx.x;
+        v[i] = q < quads ? load4(x, q) : zero;
+        o[i] = q < quads ? load4(other, q) : zero;
+        p[i] = first && q < quads ? load4(slot, q) : zero;
+    }
+#pragma unroll
+    for (int i = 0; i < VPT; ++i) {
+        ss.x += squares(v[i]);
+        ss.y += squares(o[i]);
+    }
+    ss.x = warp_sum(ss.x);
+    ss.y = warp_sum(ss.y);
+    if ((threadIdx.x & 31) == 0) of_warp[threadIdx.x >> 5] = ss;
+    __syncthreads();
+    ss = of_warp[0];
+#pragma unroll
+    for (int i = 1; i < 8; ++i) {
+        ss.x += of_warp[i].x;
+        ss.y += of_warp[i].y;
+    }
+    const float inv = 1.0f / sqrtf(ss.x / (float)hidden + eps), inv_other = 1.0f / sqrtf(ss.y / (float)hidden + eps);
+    auto mixed = [](float x, float before, float m) { return fmaf(before - x, m, x); };
+#pragma unroll
+    for (int i = 0; i < VPT; ++i) {
+        const int q = i * 256 + threadIdx.x;
+        if (q >= quads) continue;
+        const float4 n = make_float4(g[i].x * (v[i].x * inv), g[i].y * (v[i].y * inv), g[i].z * (v[i].z * inv), g[i].w * (v[i].w * inv));
+        const float4 b = make_float4(g[i].x * (o[i].x * inv_other), g[i].y * (o[i].y * inv_other), g[i].z * (o[i].z * inv_other), g[i].w * (o[i].w * inv_other));
+        const float4 before = first ? p[i] : b;
+        store4(out + (size_t)t * hidden, q, make_float4(mixed(n.x, before.x, w[i].x), mixed(n.y, before.y, w[i].y), mixed(n.z, before.z, w[i].z), mixed(n.w, before.w, w[i].w)));
+        if (first) store4(slot, q, b);
     }
 }
 
@@ -398,8 +469,23 @@ EG_API int eg_rmsnorm_shift(cudaStream_t stream, const float* residual, const fl
                             int tokens, int hidden) {
     if (tokens <= 0) return 0;
     // (few rows: a block a row spreads a row's loads over more threads; measured at 8 rows of 2,048: 8 us against 18)
-    if (tokens >= 256 && hidden % 4 == 0 && hidden <= 2048 && slot_floats % 4 == 0 && aligned16(residual) && aligned16(gain) && aligned16(mu) && aligned16(state) &&
-        aligned16(out)) {
+    const bool pieces = hidden % 4 == 0 && slot_floats % 4 == 0 && aligned16(residual) && aligned16(gain) && aligned16(mu) && aligned16(state) && aligned16(out);
+    if (tokens < 256 && pieces && hidden <= 4096) {
+#define EG_SHIFT_ROW(TO, V) \
+    eg_pdl_launch(rmsnorm_shift_row_kernel<TO, V>, tokens, 256, 0, stream, residual, gain, eps, mu, state, slot_floats, token_seq, seq_starts, seq_slots, (TO*)out, hidden)
+        if (out_dtype == EG_BF16) {
+            if (hidden <= 1024) EG_SHIFT_ROW(bf16, 1);
+            else if (hidden <= 2048) EG_SHIFT_ROW(bf16, 2);
+            else EG_SHIFT_ROW(bf16, 4);
+        } else {
+            if (hidden <= 1024) EG_SHIFT_ROW(float, 1);
+            else if (hidden <= 2048) EG_SHIFT_ROW(float, 2);
+            else EG_SHIFT_ROW(float, 4);
+        }
+#undef EG_SHIFT_ROW
+        return eg_launch_status();
+    }
+    if (tokens >= 256 && hidden <= 2048 && pieces) {
         // four warps a block: 512 blocks at 2,048 rows, all resident at once (measured cold: 16.5 us a launch; eight warps a block 17.1)
         const int nt = 128, blocks = (tokens + 3) / 4;
         const int vpl = (hidden / 4 + 31) / 32;
@@ -435,17 +521,19 @@ EG_API int eg_rmsnorm_add(cudaStream_t stream, float* residual, const void* y, i
         int blocks, nt;
         warp_rows_launch(tokens, &blocks, &nt);
         const int vpl = (hidden / 4 + 31) / 32;
-#define EG_ADD_WARP(TD, V) eg_pdl_launch(rmsnorm_add_warp_kernel<TD, V>, blocks, nt, 0, stream, residual, (const TD*)y, ldy, gain, eps, tokens, hidden)
+#define EG_ADD_WARP(TD, V)                                                                                                                              \
+    if (nt == 32 && V <= 16) eg_pdl_launch(rmsnorm_add_warp_kernel<TD, V, V <= 16>, blocks, nt, 0, stream, residual, (const TD*)y, ldy, gain, eps, tokens, hidden); \
+    else eg_pdl_launch(rmsnorm_add_warp_kernel<TD, V, false>, blocks, nt, 0, stream, residual, (const TD*)y, ldy, gain, eps, tokens, hidden)
         if (y_dtype == EG_BF16) {
-            if (vpl <= 4) EG_ADD_WARP(bf16, 4);
-            else if (vpl <= 8) EG_ADD_WARP(bf16, 8);
-            else if (vpl <= 16) EG_ADD_WARP(bf16, 16);
-            else EG_ADD_WARP(bf16, 32);
+            if (vpl <= 4) { EG_ADD_WARP(bf16, 4); }
+            else if (vpl <= 8) { EG_ADD_WARP(bf16, 8); }
+            else if (vpl <= 16) { EG_ADD_WARP(bf16, 16); }
+            else { EG_ADD_WARP(bf16, 32); }
         } else {
-            if (vpl <= 4) EG_ADD_WARP(float, 4);
-            else if (vpl <= 8) EG_ADD_WARP(float, 8);
-            else if (vpl <= 16) EG_ADD_WARP(float, 16);
-            else EG_ADD_WARP(float, 32);
+            if (vpl <= 4) { EG_ADD_WARP(float, 4); }
+            else if (vpl <= 8) { EG_ADD_WARP(float, 8); }
+            else if (vpl <= 16) { EG_ADD_WARP(float, 16); }
+            else { EG_ADD_WARP(float, 32); }
         }
 #undef EG_ADD_WARP
         return eg_launch_status();

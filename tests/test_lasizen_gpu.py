@@ -421,3 +421,40 @@ def test_command_line_with_random_weights(tmp_path):
         for i, tok in enumerate(out):
             row = logits[len(prompt) + i - 1]
             assert float(row.max() - row[tok]) <= 4e-4 * np.abs(row).max(), (i, tok, int(row.argmax()))
+
+
+@pytest.mark.parametrize("hidden", [20, 1024, 1028, 2052, 4096, 1022])
+@pytest.mark.parametrize("entries", [[1, 1, 1], [3, 1, 40]])
+def test_norm_and_shift_of_few_rows(hidden, entries):
+    """The kernel that a row has a block of its own in (and the general one, for rows that are no whole pieces of four): against
+    norm, shift and the slots' new rows one by one."""
+    import ctypes
+
+    import torch
+
+    from easy_gpt.cpp_b200 import kernels
+
+    T, n, slots = sum(entries), len(entries), [2, 0, 3]
+    g = torch.Generator().manual_seed(hidden + T)
+    x, gain, mu = torch.randn(T, hidden, generator=g) * 3, 1 + 0.1 * torch.randn(hidden, generator=g), torch.rand(hidden, generator=g)
+    state = torch.randn(4, hidden + 4, generator=g)
+    starts = torch.tensor([0, *np.cumsum(entries)], dtype=torch.int32)
+    seq = torch.repeat_interleave(torch.arange(n, dtype=torch.int32), torch.tensor(entries))
+    normed = (x.double() / torch.sqrt((x.double() ** 2).mean(1, keepdim=True) + 1e-6)) * gain.double()
+    want, want_state = torch.empty(T, hidden, dtype=torch.float64), state.double().clone()
+    for e in range(n):
+        lo, hi = int(starts[e]), int(starts[e + 1])
+        before = torch.cat([state[slots[e], :hidden].double()[None], normed[lo:hi - 1]])
+        want[lo:hi] = normed[lo:hi] + (before - normed[lo:hi]) * mu.double()
+        want_state[slots[e], :hidden] = normed[hi - 1]
+    d = [t.cuda() for t in (x, gain, mu, state, seq, starts, torch.tensor(slots, dtype=torch.int32))]
+    out = torch.empty(T, hidden, device="cuda")
+    p = [ctypes.c_void_p(t.data_ptr()) for t in d]
+    fn = kernels.library().eg_rmsnorm_shift
+    fn.restype = ctypes.c_int
+    code = fn(ctypes.c_void_p(torch.cuda.current_stream().cuda_stream), p[0], p[1], ctypes.c_float(1e-6), p[2], p[3], ctypes.c_longlong(hidden + 4), p[4], p[5],
+              p[6], ctypes.c_void_p(out.data_ptr()), ctypes.c_int(0), ctypes.c_int(T), ctypes.c_int(hidden))
+    assert code == 0
+    # float32 sums of `hidden` squares and four roundings behind them
+    assert float((out.cpu().double() - want).abs().max()) <= 2e-6 * float(want.abs().max())
+    assert float((d[3].cpu().double() - want_state).abs().max()) <= 2e-6 * float(want_state.abs().max())
