@@ -202,13 +202,16 @@ f32_rows_kernel(const float* __restrict__ A, int lda, const float* __restrict__ 
     cluster.sync();                   // nobody leaves while another reads its sums
 }
 
-// 256 threads; thread (tx, ty) has tokens ty * TM .. + TM and rows tx * 4 .. + 4 and 64 + tx * 4 .. + 4 of a tile.
+// Thread (tx, ty) has tokens ty * 8 .. + 8 and rows tx * 4 .. + 4 and 64 + tx * 4 .. + 4 of a tile: what bounds the kernel are
+// the loads from shared memory, and 64 results a thread take four of them for 32 packed products (with 32 results a thread,
+// three for 16, 350 tokens of the 0.5B sizes took 118 us a product in the mean, this 100; pairs of rows against inputs
+// stored twice, four loads for 16 products, 141).
 template <int BM, bool VEC>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(BM * 2)
 f32_tile_kernel(const float* __restrict__ A, int lda, const float* __restrict__ W, int ldw, const float* __restrict__ bias, float* __restrict__ C, int ldc,
                 int M, int N, int K, int part_len, int groups, int split) {
-    constexpr int TM = BM / 16, A_STRIDE = BM + 4, N_STRIDE = BN + 4;
-    constexpr int A_LOADS = BM * BK / 4 / 256, W_LOADS = BN * BK / 4 / 256;
+    constexpr int THREADS = BM * 2, PASS = THREADS / 4, TM = 8, A_STRIDE = BM + 4, N_STRIDE = BN + 4;
+    constexpr int A_LOADS = BM / PASS, W_LOADS = BN / PASS;
     extern __shared__ __align__(16) float smem[];
     float* As = smem;                                  // [2][BK][A_STRIDE]
     float* Ws = smem + 2 * BK * A_STRIDE;              // [2][BK][N_STRIDE]
@@ -230,26 +233,26 @@ f32_tile_kernel(const float* __restrict__ A, int lda, const float* __restrict__ 
             return v;
         };
 #pragma unroll
-        for (int i = 0; i < A_LOADS; ++i) a_next[i] = piece(A, lda, m0 + i * 64 + tid / 4, M, k0 + tid % 4 * 4);
+        for (int i = 0; i < A_LOADS; ++i) a_next[i] = piece(A, lda, m0 + i * PASS + tid / 4, M, k0 + tid % 4 * 4);
 #pragma unroll
-        for (int i = 0; i < W_LOADS; ++i) w_next[i] = piece(W, ldw, n0 + i * 64 + tid / 4, N, k0 + tid % 4 * 4);
+        for (int i = 0; i < W_LOADS; ++i) w_next[i] = piece(W, ldw, n0 + i * PASS + tid / 4, N, k0 + tid % 4 * 4);
     };
     auto put = [&](int buffer) {
         float* as = As + buffer * BK * A_STRIDE + tid % 4 * 4 * A_STRIDE + tid / 4;
         float* ws = Ws + buffer * BK * N_STRIDE + tid % 4 * 4 * N_STRIDE + tid / 4;
 #pragma unroll
         for (int i = 0; i < A_LOADS; ++i) {
-            as[i * 64] = a_next[i].x;
-            as[A_STRIDE + i * 64] = a_next[i].y;
-            as[2 * A_STRIDE + i * 64] = a_next[i].z;
-            as[3 * A_STRIDE + i * 64] = a_next[i].w;
+            as[i * PASS] = a_next[i].x;
+            as[A_STRIDE + i * PASS] = a_next[i].y;
+            as[2 * A_STRIDE + i * PASS] = a_next[i].z;
+            as[3 * A_STRIDE + i * PASS] = a_next[i].w;
         }
 #pragma unroll
         for (int i = 0; i < W_LOADS; ++i) {
-            ws[i * 64] = w_next[i].x;
-            ws[N_STRIDE + i * 64] = w_next[i].y;
-            ws[2 * N_STRIDE + i * 64] = w_next[i].z;
-            ws[3 * N_STRIDE + i * 64] = w_next[i].w;
+            ws[i * PASS] = w_next[i].x;
+            ws[N_STRIDE + i * PASS] = w_next[i].y;
+            ws[2 * N_STRIDE + i * PASS] = w_next[i].z;
+            ws[3 * N_STRIDE + i * PASS] = w_next[i].w;
         }
     };
 
@@ -341,7 +344,7 @@ f32_tile_kernel(const float* __restrict__ A, int lda, const float* __restrict__ 
         }
     cg::cluster_group cluster = cg::this_cluster();
     cluster.sync();
-    for (int e = my_group * 256 + tid; e < BM * BN; e += groups * 256) {
+    for (int e = my_group * THREADS + tid; e < BM * BN; e += groups * THREADS) {
         const int m = m0 + e / BN, n = n0 + e % BN;
         if (m >= M || n >= N) continue;
         float part[MAX_GROUPS];
@@ -396,12 +399,12 @@ int launch_f32(cudaStream_t stream, const float* A, int lda, const float* W, int
     const long long columns = (N + BN - 1) / BN;
     if (columns * ((M + 127) / 128) >= 296) {
         constexpr int smem = 2 * BK * (128 + 4 + BN + 4) * 4;
-        return launch_clusters(f32_tile_kernel<128, VEC>, dim3((unsigned)columns, (M + 127) / 128), 256, smem, 1, stream, A, lda, W, ldw, bias, C, ldc, M, N, K,
+        return launch_clusters(f32_tile_kernel<128, VEC>, dim3((unsigned)columns, (M + 127) / 128), 2 * 128, smem, 1, stream, A, lda, W, ldw, bias, C, ldc, M, N, K,
                                cut.part_len, cut.groups, 0);
     }
     const int split = cut.groups > 1 && columns * ((M + 63) / 64) < 296;
     constexpr int tile_bytes = 2 * BK * (64 + 4 + BN + 4) * 4, sums_bytes = 64 * BN * 4;
-    return launch_clusters(f32_tile_kernel<64, VEC>, dim3((unsigned)columns * (split ? cut.groups : 1), (M + 63) / 64), 256,
+    return launch_clusters(f32_tile_kernel<64, VEC>, dim3((unsigned)columns * (split ? cut.groups : 1), (M + 63) / 64), 2 * 64,
                            tile_bytes > sums_bytes ? tile_bytes : sums_bytes, split ? cut.groups : 1, stream, A, lda, W, ldw, bias, C, ldc, M, N, K, cut.part_len,
                            cut.groups, split);
 }
