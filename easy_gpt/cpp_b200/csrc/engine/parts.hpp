@@ -44,7 +44,7 @@ inline DeviceBuffer upload(const StoredTensor& t, DType dtype) {
 }
 
 // ---- y = x W^T + b with W stored [out, in] (src/models/linear.cpp:42-44) ------------------------------------------
-// In bfloat16, steps of up to 16 tokens go to the engine's own weight-streaming kernel (gemm_skinny.cu); larger ones
+// In bfloat16, steps of up to 16 tokens go to the engine's own weight-streaming kernels (gemm_stream.cu, gemm_skinny.cu); larger ones
 // to the library product (cuBLAS), where the reference's engine calls cublasGemmEx too (src/cuda/ops/matmul.cu:194-204).
 // In float32 it is always the engine's own FFMA kernel: true 32-bit arithmetic whose sums do not depend on the batch.
 struct SkinnyRope {

@@ -109,6 +109,7 @@ struct SkinnyPlan {
     int row_blocks, k_slices, k_split;
 };
 // How the warps of a CTA and the CTAs of the grid share a [n_rows, in_features] weight matrix.
+// (The register-fed kernel's plan, and how many rows a partial sum of squares stands for; gemm_stream.cu has a plan of its own.)
 inline SkinnyPlan skinny_plan(int n_rows, int in_features, int head_dim = 0) {
     const int chunks = (in_features + 63) / 64;
     if (head_dim) {                                    // fused QKV: one CTA per head
