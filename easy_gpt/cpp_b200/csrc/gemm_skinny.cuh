@@ -6,6 +6,8 @@ namespace skinny {
 
 enum { EPI_STORE = 0, EPI_F32 = 1, EPI_SWIGLU = 2, EPI_QKV_ROPE = 3, EPI_RESID_NORM = 4 };
 
+constexpr unsigned WAIT_LIMIT = 1u << 22;    // polls of a wait in gemm_stream.cu
+
 struct Params {
     const bf16* W;
     long long ldw;
@@ -51,6 +53,7 @@ struct Params {
     int* counters;               // [gridDim.x] tickets, zero before and after every launch
     unsigned long long* trace;   // optional: [2] earliest start / latest end of this launch's CTAs (%globaltimer, ns)
     int parts_offset;            // where in shared memory the cluster's parts arrive (bytes)
+    unsigned wait_limit;         // gemm_stream.cu: polls after which a wait for weights or a free stage gives up (at most WAIT_LIMIT)
     int cluster_reduce;          // the gridDim.y CTAs of a row group are one cluster and sum their parts through the first one's shared memory
 };
 

@@ -34,7 +34,6 @@ constexpr int PREFETCH_PIECE = 16 * 1024;
 constexpr int SMS = 148;                       // a constant, so that results do not hang off the GPU
 constexpr int WIDE_BLOCKS = 400;              // row blocks from which on CTAs read all of K
 constexpr int MOST_SHARED = 220 * 1024;
-constexpr unsigned WAIT_LIMIT = 1u << 22;
 
 struct Plan {
     int rb_log;                               // log2 of a unit's row blocks; the other factor of WARPS are slices of K, each one tile of a stage
@@ -63,8 +62,8 @@ __device__ __forceinline__ bool try_wait_cluster(uint64_t* bar, uint32_t parity)
     return ok != 0;
 }
 // mbar_wait_bounded for launches that may come without a status word
-__device__ __forceinline__ bool wait_for(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int* status) {
-    for (unsigned i = 0; i < WAIT_LIMIT; ++i) {
+__device__ __forceinline__ bool wait_for(uint64_t* bar, uint32_t parity, unsigned limit, volatile int* abort_flag, int* status) {
+    for (unsigned i = 0; i < limit; ++i) {
         if (mbar_try_wait(bar, parity)) return true;
         if (*abort_flag) return false;
     }
@@ -83,7 +82,7 @@ stream_kernel(const Params p, const Plan s, const __grid_constant__ CUtensorMap 
     unsigned char* smem = smem_raw + ((1024u - (smem_addr(smem_raw) & 1023u)) & 1023u);      // swizzled tiles start on 1,024 bytes
     __shared__ __align__(8) uint64_t full[MAX_STAGES], empty[MAX_STAGES], factor_bar, parts_bar;
     __shared__ float factor[MT];
-    __shared__ volatile int abort_flag;
+    __shared__ volatile int abort_flag, asked;                    // asked: stages that the copying warp has asked for, once it is done
     TraceScope trace_scope(p.trace);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const bool clustered = gridDim.y > 1;
@@ -117,6 +116,7 @@ stream_kernel(const Params p, const Plan s, const __grid_constant__ CUtensorMap 
         mbar_init(&factor_bar, 1);
         mbar_init(&parts_bar, 1);
         abort_flag = 0;
+        asked = -1;
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
         if (clustered && blockIdx.y == 0) mbar_expect_tx(&parts_bar, (gridDim.y - 1) * (uint32_t)rows_per_unit * (uint32_t)p.M * 4u);
     }
@@ -183,14 +183,13 @@ stream_kernel(const Params p, const Plan s, const __grid_constant__ CUtensorMap 
         }
         bool ok = true;
         for (uint32_t phase = 0; ok && issued < total;) {
-            ok = wait_for(&empty[in_slot], phase, &abort_flag, p.status);
+            // (a warp that gave up a wait for weights leaves its stages unread: a stage that is free may still be being filled)
+            ok = wait_for(&empty[in_slot], phase, p.wait_limit, &abort_flag, p.status) && !abort_flag;
             ok = __all_sync(0xffffffffu, ok);
             if (ok) issue();
             if (in_slot == 0) phase ^= 1u;
         }
-        if (!ok)                                                  // gave up: nothing leaves while its copies are in flight
-            for (int it = max(0, issued - s.stages); it < issued; ++it)
-                for (unsigned i = 0; i < WAIT_LIMIT && !mbar_try_wait(&full[it % s.stages], (uint32_t)(it / s.stages) & 1u); ++i) {}
+        if (lane == 0) asked = issued;
         return;
     }
 
@@ -261,13 +260,23 @@ stream_kernel(const Params p, const Plan s, const __grid_constant__ CUtensorMap 
         w_step[j] = smem_addr(smem) + ks * tile_bytes + (uint32_t)(rb * 16 + (lane & 15)) * 128 + (((j * 2 + (lane >> 4)) ^ (lane & 7)) << 4);
     int slot = 0;
     uint32_t phase = 0;
+    // Nothing leaves while copies are on their way: a warp that has waited for every stage has seen all of them land, and one
+    // that gave up waits here (with a limit) for the last copy of each stage.
+    auto leave = [&]() {
+        if (ok) return;
+        unsigned left = WAIT_LIMIT;
+        while (asked < 0 && --left) {}
+        const int issued_in_all = max(0, asked), open = min(s.stages, issued_in_all);
+        for (int it = issued_in_all - open; it < issued_in_all; ++it)
+            while (left && !mbar_try_wait(&full[it % s.stages], (uint32_t)(it / s.stages) & 1u)) --left;
+    };
     for (int unit = 0; unit < units; ++unit) {
         const int rows = rows_of(unit);
         float acc[NT][4];
 #pragma unroll
         for (int i = 0; i < NT; ++i) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.f;
         for (int st = 0; st < k_stages; ++st) {
-            ok = ok && wait_for(&full[slot], phase, &abort_flag, p.status);
+            ok = ok && wait_for(&full[slot], phase, p.wait_limit, &abort_flag, p.status);
             const int k = st * kc + ks * 64;
             if (rb * 16 < rows && k < k_len) {
                 // all loads of the tile first: the products then follow one another without a trip to shared memory between them
@@ -302,7 +311,7 @@ stream_kernel(const Params p, const Plan s, const __grid_constant__ CUtensorMap 
         }
         if (unit == 0) {
             trace_scope.mark(3, true);
-            if (NORM == 2) ok = ok && wait_for(&factor_bar, 0, &abort_flag, p.status);
+            if (NORM == 2) ok = ok && wait_for(&factor_bar, 0, p.wait_limit, &abort_flag, p.status);
         } else {
             consumers_sync();                                     // the unit in front has been read
         }
@@ -336,6 +345,7 @@ stream_kernel(const Params p, const Plan s, const __grid_constant__ CUtensorMap 
                 for (int e = threadIdx.x; e < elems; e += WARPS * 32)
                     asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b32 [%0], %1, [%2];\n"
                                  ::"r"(to + (uint32_t)e * 4u), "r"(__float_as_uint(slices(e & (rows_per_unit - 1), e >> row_log))), "r"(bar) : "memory");
+                leave();
                 return;
             }
             // this CTA's own sum first, then the others', in their order; into the first slice's place
@@ -343,8 +353,11 @@ stream_kernel(const Params p, const Plan s, const __grid_constant__ CUtensorMap 
                 const int m = e >> row_log, r = e & (rows_per_unit - 1);
                 red[((r >> 4) * MT + m) * RED_LD + (r & 15)] = slices(r, m);
             }
+            // (The others send their parts whatever became of their own waits, at most one limit a stage later: this CTA must
+            // not be gone by then.)
             bool landed = false;
-            for (unsigned i = 0; i < WAIT_LIMIT && !landed; ++i) landed = try_wait_cluster(&parts_bar, 0);
+            for (int st = 0; st < s.k_stages + 2 && !landed; ++st)
+                for (unsigned i = 0; i < WAIT_LIMIT && !landed; ++i) landed = try_wait_cluster(&parts_bar, 0);
             if (!landed && p.status) atomicOr(p.status, EG_STATUS_WAIT_TIMEOUT);
             for (int e = threadIdx.x; e < elems; e += WARPS * 32) {
                 const int m = e >> row_log, r = e & (rows_per_unit - 1);
@@ -427,6 +440,7 @@ stream_kernel(const Params p, const Plan s, const __grid_constant__ CUtensorMap 
             }
         }
     }
+    leave();
 }
 
 namespace {

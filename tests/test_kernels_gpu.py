@@ -700,6 +700,25 @@ def test_gemm_stream_units_splits_and_shares(M, N, K):
     assert float((out.cpu() - want).abs().max()) <= 1e-5 * float(want.abs().max()) * math.sqrt(K)       # float32 accumulation
 
 
+@pytest.mark.parametrize("M", [1, 16])
+@pytest.mark.parametrize("N, K", [(48, 80), (896, 896), (896, 4864), (200, 2064), (6416, 2064), (19001, 896)])
+def test_gemm_stream_whose_waits_give_up_leaves_nothing_behind(M, N, K):
+    """Waits that give up at their first poll, while the weights are on their way: all stages asked for at once and a ring that
+    would go round, one CTA and clusters, one unit and shares.  The kernel says so and returns, and the next launches are right."""
+    from easy_gpt.cpp_b200 import kernels
+
+    x, w = bf(torch.randn(M, K, generator=gen(90))).to(DEV), bf(torch.randn(N, K, generator=gen(91)) * 0.1).to(DEV)
+    status = torch.zeros(1, dtype=torch.int32, device=DEV)
+    before, after, lost = (torch.empty(M, N, device=DEV) for _ in range(3))
+    kernels.gemm_skinny(w, None, before, kernels.EPI_F32, x=x, kernel=1, status=status)
+    assert status.item() == 0
+    for _ in range(20):
+        kernels.gemm_skinny(w, None, lost, kernels.EPI_F32, x=x, kernel=1, wait_limit=0, status=status)
+    kernels.gemm_skinny(w, None, after, kernels.EPI_F32, x=x, kernel=1)
+    assert status.item() == 8
+    assert torch.equal(before, after)
+
+
 @pytest.mark.parametrize("M, H, I, J", [(1, 896, 4864, 4864), (16, 208, 2064, 9600), (9, 1040, 304, 72)])
 def test_gemm_stream_residual_norm_then_swiglu(M, H, I, J):
     from easy_gpt.cpp_b200 import kernels
