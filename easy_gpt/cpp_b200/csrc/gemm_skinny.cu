@@ -655,7 +655,7 @@ static int gemm_skinny_any(cudaStream_t stream, int epilogue, int norm, int use_
                            long long head_stride, long long pool_slots, int* status, const void* prefetch,
                            long long prefetch_bytes, unsigned long long* trace, const float* ss_in, int ss_parts,
                            float* resid_inout, const float* gain_out, void* xn_out, float* ss_out, int act, float act_a, float act_b,
-                           int kernel = 0, unsigned wait_limit = skinny::WAIT_LIMIT) {
+                           int kernel = 0, int give_up = 0) {
     if (M <= 0 || N <= 0) return 0;
     if (norm < 0 || norm > 2 || (norm == 2 && (!delta || !ss_in || ss_parts < 1)) ||
         (epilogue == EPI_RESID_NORM && (!resid_inout || !gain_out || !xn_out || !ss_out)))
@@ -679,7 +679,7 @@ static int gemm_skinny_any(cudaStream_t stream, int epilogue, int norm, int use_
     p.norm_mode = norm; p.ss_in = ss_in; p.ss_parts = ss_parts;
     p.resid_inout = resid_inout; p.gain_out = gain_out; p.xn_out = (bf16*)xn_out; p.ss_out = ss_out;
     p.act = act; p.act_a = act_a; p.act_b = act_b;
-    p.wait_limit = wait_limit;
+    p.give_up = give_up;
     const int taken = kernel == 2 ? -1 : eg_gemm_stream_launch(stream, epilogue, norm, p);
     if (taken >= 0) return taken;
     if (kernel == 1) return (int)cudaErrorInvalidValue;
@@ -714,9 +714,9 @@ EG_API int eg_gemm_skinny(cudaStream_t stream, int epilogue, int norm, int use_p
 }
 
 // eg_gemm_skinny on a kernel of the caller's choice, for tests and measurements: 1 gemm_stream.cu's (refused where that does not take the
-// sizes), 2 this file's, 0 as eg_gemm_skinny chooses.  wait_limit: polls after which a wait inside gemm_stream.cu's kernel gives up, sets
-// EG_STATUS_WAIT_TIMEOUT and leaves the result undefined (0: at once; at most 2^22, what the products run with).
-EG_API int eg_gemm_decode(int kernel, unsigned wait_limit, cudaStream_t stream, int epilogue, int norm, int use_pdl, const void* W, long long ldw,
+// sizes), 2 this file's, 0 as eg_gemm_skinny chooses.  With give_up (kernel 1, EPI_F32 of plain rows) the waits inside the kernel are as if
+// they had run out at once: EG_STATUS_WAIT_TIMEOUT is set and the result undefined.
+EG_API int eg_gemm_decode(int kernel, int give_up, cudaStream_t stream, int epilogue, int norm, int use_pdl, const void* W, long long ldw,
                           const float* bias, int M, int N, int K, const void* x, long long ldx, const float* resid_in,
                           float* resid_out, const void* delta, const float* gain, float eps, void* out, long long ldo,
                           int row_blocks, int k_slices, int k_split, float* scratch, int* counters, int num_heads,
@@ -725,11 +725,11 @@ EG_API int eg_gemm_decode(int kernel, unsigned wait_limit, cudaStream_t stream, 
                           long long head_stride, long long pool_slots, int* status, const void* prefetch,
                           long long prefetch_bytes, unsigned long long* trace, const float* ss_in, int ss_parts,
                           float* resid_inout, const float* gain_out, void* xn_out, float* ss_out) {
-    if (kernel < 0 || kernel > 2 || wait_limit > skinny::WAIT_LIMIT) return (int)cudaErrorInvalidValue;
+    if (kernel < 0 || kernel > 2 || (give_up && (kernel != 1 || epilogue != EPI_F32 || norm))) return (int)cudaErrorInvalidValue;
     return gemm_skinny_any(stream, epilogue, norm, use_pdl, W, ldw, bias, M, N, K, x, ldx, resid_in, resid_out, delta, gain, eps, out, ldo, row_blocks,
                            k_slices, k_split, scratch, counters, num_heads, num_kv_heads, head_dim, positions, slot_map, k_cache, v_cache, inv_freq,
                            page_size, page_stride, head_stride, pool_slots, status, prefetch, prefetch_bytes, trace, ss_in, ss_parts, resid_inout,
-                           gain_out, xn_out, ss_out, 0, 0.f, 0.f, kernel, wait_limit);
+                           gain_out, xn_out, ss_out, 0, 0.f, 0.f, kernel, give_up);
 }
 
 // out [M, N] bfloat16 = act(x W^T) with the xIELU activation applied to the finished sums: act(z) = act_a z^2 + z / 2 for

@@ -34,7 +34,10 @@ struct Params {
     int* status;
     int RB, KS;
     int use_pdl;
-    int stage_norm;              // the norm prologue's input comes through one bulk copy into shared memory
+    union {
+        int stage_norm;          // gemm_skinny.cu: the norm prologue's input comes through one bulk copy into shared memory
+        int give_up;             // gemm_stream.cu, for tests (EPI_F32 of plain rows): every wait inside the kernel gives up at once
+    };
     int norm_mode;               // 1: add + norm here; 2: prenormed rows (delta = xn) and partial sums (ss_in)
     const float* ss_in;          // [ss_parts][padded tokens] partial sums of squares, prenormed prologue
     int ss_parts;
@@ -53,7 +56,6 @@ struct Params {
     int* counters;               // [gridDim.x] tickets, zero before and after every launch
     unsigned long long* trace;   // optional: [2] earliest start / latest end of this launch's CTAs (%globaltimer, ns)
     int parts_offset;            // where in shared memory the cluster's parts arrive (bytes)
-    unsigned wait_limit;         // gemm_stream.cu: polls after which a wait for weights or a free stage gives up (at most WAIT_LIMIT)
     int cluster_reduce;          // the gridDim.y CTAs of a row group are one cluster and sum their parts through the first one's shared memory
 };
 

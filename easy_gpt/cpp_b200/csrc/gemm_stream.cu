@@ -34,6 +34,7 @@ constexpr int PREFETCH_PIECE = 16 * 1024;
 constexpr int SMS = 148;                       // a constant, so that results do not hang off the GPU
 constexpr int WIDE_BLOCKS = 400;              // row blocks from which on CTAs read all of K
 constexpr int MOST_SHARED = 220 * 1024;
+constexpr unsigned PARTS_WAIT_LIMIT = WAIT_LIMIT << 7;
 
 struct Plan {
     int rb_log;                               // log2 of a unit's row blocks; the other factor of WARPS are slices of K, each one tile of a stage
@@ -62,8 +63,8 @@ __device__ __forceinline__ bool try_wait_cluster(uint64_t* bar, uint32_t parity)
     return ok != 0;
 }
 // mbar_wait_bounded for launches that may come without a status word
-__device__ __forceinline__ bool wait_for(uint64_t* bar, uint32_t parity, unsigned limit, volatile int* abort_flag, int* status) {
-    for (unsigned i = 0; i < limit; ++i) {
+__device__ __forceinline__ bool wait_for(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int* status) {
+    for (unsigned i = 0; i < WAIT_LIMIT; ++i) {
         if (mbar_try_wait(bar, parity)) return true;
         if (*abort_flag) return false;
     }
@@ -74,7 +75,8 @@ __device__ __forceinline__ bool wait_for(uint64_t* bar, uint32_t parity, unsigne
 __device__ __forceinline__ void consumers_sync() { asm volatile("bar.sync 1, %0;\n" ::"n"(WARPS * 32) : "memory"); }
 }  // namespace
 
-template <int NT, int EPI, int NORM>
+// GIVE_UP, for tests: every wait inside the kernel is as if it had run out at once
+template <int NT, int EPI, int NORM, bool GIVE_UP>
 __global__ void __launch_bounds__(THREADS, 2)
 stream_kernel(const Params p, const Plan s, const __grid_constant__ CUtensorMap unit_map, const __grid_constant__ CUtensorMap block_map) {
     constexpr int MT = NT * 8;
@@ -115,7 +117,7 @@ stream_kernel(const Params p, const Plan s, const __grid_constant__ CUtensorMap 
         }
         mbar_init(&factor_bar, 1);
         mbar_init(&parts_bar, 1);
-        abort_flag = 0;
+        abort_flag = GIVE_UP;
         asked = -1;
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
         if (clustered && blockIdx.y == 0) mbar_expect_tx(&parts_bar, (gridDim.y - 1) * (uint32_t)rows_per_unit * (uint32_t)p.M * 4u);
@@ -181,10 +183,9 @@ stream_kernel(const Params p, const Plan s, const __grid_constant__ CUtensorMap 
             __syncwarp();
             if (lane == 0) mbar_arrive(&factor_bar);
         }
-        bool ok = true;
+        bool ok = !GIVE_UP;
         for (uint32_t phase = 0; ok && issued < total;) {
-            // (a warp that gave up a wait for weights leaves its stages unread: a stage that is free may still be being filled)
-            ok = wait_for(&empty[in_slot], phase, p.wait_limit, &abort_flag, p.status) && !abort_flag;
+            ok = wait_for(&empty[in_slot], phase, &abort_flag, p.status);
             ok = __all_sync(0xffffffffu, ok);
             if (ok) issue();
             if (in_slot == 0) phase ^= 1u;
@@ -247,7 +248,7 @@ stream_kernel(const Params p, const Plan s, const __grid_constant__ CUtensorMap 
     }
     cp_async_wait<0>();
     consumers_sync();
-    bool ok = true;
+    bool ok = !GIVE_UP;
     trace_scope.mark(2);
 
     float* red = reinterpret_cast<float*>(smem + s.red_offset);              // [WARPS][MT][RED_LD]
@@ -264,10 +265,11 @@ stream_kernel(const Params p, const Plan s, const __grid_constant__ CUtensorMap 
     // that gave up waits here (with a limit) for the last copy of each stage.
     auto leave = [&]() {
         if (ok) return;
+        if (p.status) atomicOr(p.status, EG_STATUS_WAIT_TIMEOUT);
         unsigned left = WAIT_LIMIT;
         while (asked < 0 && --left) {}
-        const int issued_in_all = max(0, asked), open = min(s.stages, issued_in_all);
-        for (int it = issued_in_all - open; it < issued_in_all; ++it)
+        const int in_all = max(0, asked);
+        for (int it = max(0, in_all - s.stages); it < in_all; ++it)
             while (left && !mbar_try_wait(&full[it % s.stages], (uint32_t)(it / s.stages) & 1u)) --left;
     };
     for (int unit = 0; unit < units; ++unit) {
@@ -276,7 +278,7 @@ stream_kernel(const Params p, const Plan s, const __grid_constant__ CUtensorMap 
 #pragma unroll
         for (int i = 0; i < NT; ++i) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.f;
         for (int st = 0; st < k_stages; ++st) {
-            ok = ok && wait_for(&full[slot], phase, p.wait_limit, &abort_flag, p.status);
+            ok = ok && wait_for(&full[slot], phase, &abort_flag, p.status);
             const int k = st * kc + ks * 64;
             if (rb * 16 < rows && k < k_len) {
                 // all loads of the tile first: the products then follow one another without a trip to shared memory between them
@@ -306,12 +308,12 @@ stream_kernel(const Params p, const Plan s, const __grid_constant__ CUtensorMap 
                         for (int nt = 0; nt < NT; ++nt) mma_bf16_16816(acc[nt], a[j], b[j][nt][0], b[j][nt][1]);
             }
             __syncwarp();
-            if (lane == 0) mbar_arrive(&empty[slot]);
+            if (lane == 0 && ok) mbar_arrive(&empty[slot]);       // (who gave up has not seen the stage full: it is not asked for again)
             if (++slot == s.stages) { slot = 0; phase ^= 1u; }
         }
         if (unit == 0) {
             trace_scope.mark(3, true);
-            if (NORM == 2) ok = ok && wait_for(&factor_bar, 0, p.wait_limit, &abort_flag, p.status);
+            if (NORM == 2) ok = ok && wait_for(&factor_bar, 0, &abort_flag, p.status);
         } else {
             consumers_sync();                                     // the unit in front has been read
         }
@@ -353,11 +355,10 @@ stream_kernel(const Params p, const Plan s, const __grid_constant__ CUtensorMap 
                 const int m = e >> row_log, r = e & (rows_per_unit - 1);
                 red[((r >> 4) * MT + m) * RED_LD + (r & 15)] = slices(r, m);
             }
-            // (The others send their parts whatever became of their own waits, at most one limit a stage later: this CTA must
-            // not be gone by then.)
+            // (The others send their parts whatever became of their own waits, at most one limit a stage later: this CTA
+            // must not be gone by then.)
             bool landed = false;
-            for (int st = 0; st < s.k_stages + 2 && !landed; ++st)
-                for (unsigned i = 0; i < WAIT_LIMIT && !landed; ++i) landed = try_wait_cluster(&parts_bar, 0);
+            for (unsigned i = 0; i < PARTS_WAIT_LIMIT && !landed; ++i) landed = try_wait_cluster(&parts_bar, 0);
             if (!landed && p.status) atomicOr(p.status, EG_STATUS_WAIT_TIMEOUT);
             for (int e = threadIdx.x; e < elems; e += WARPS * 32) {
                 const int m = e >> row_log, r = e & (rows_per_unit - 1);
@@ -444,7 +445,7 @@ stream_kernel(const Params p, const Plan s, const __grid_constant__ CUtensorMap 
 }
 
 namespace {
-template <int NT, int EPI, int NORM>
+template <int NT, int EPI, int NORM, bool GIVE_UP = false>
 int launch(cudaStream_t stream, const Params& p) {
     constexpr int MT = NT * 8;
     Plan s{};
@@ -515,7 +516,7 @@ int launch(cudaStream_t stream, const Params& p) {
                    CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
             return -1;
     }
-    auto kernel = stream_kernel<NT, EPI, NORM>;
+    auto kernel = stream_kernel<NT, EPI, NORM, GIVE_UP>;
     static const cudaError_t configured = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, MOST_SHARED);
     if (configured != cudaSuccess) return (int)configured;
     cudaLaunchConfig_t cfg = {};
@@ -552,6 +553,8 @@ int launch(cudaStream_t stream, const Params& p) {
 
 template <int EPI, int NORM>
 int launch_nt(cudaStream_t stream, const Params& p) {
+    if constexpr (EPI == EPI_F32 && NORM == 0)
+        if (p.give_up) return p.M <= 8 ? launch<1, EPI, NORM, true>(stream, p) : p.M <= 16 ? launch<2, EPI, NORM, true>(stream, p) : -1;
     if (p.M <= 8) return launch<1, EPI, NORM>(stream, p);
     if (p.M <= 16) return launch<2, EPI, NORM>(stream, p);
     return -1;

@@ -11,7 +11,7 @@ from __future__ import annotations
 import ctypes
 import functools
 import os
-from ctypes import c_float, c_int, c_longlong, c_uint, c_void_p
+from ctypes import c_float, c_int, c_longlong, c_void_p
 from typing import Optional
 
 import torch
@@ -84,7 +84,7 @@ class _Signatures:
                       c_void_p, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_longlong,
                       c_longlong, c_longlong, c_void_p, c_void_p, c_longlong, c_void_p, c_void_p, c_int, c_void_p, c_void_p,
                       c_void_p, c_void_p]
-    eg_gemm_decode = [c_int, c_uint, *eg_gemm_skinny]
+    eg_gemm_decode = [c_int, c_int, *eg_gemm_skinny]
     eg_gemm_tcgen05 = [c_void_p, c_int, c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_void_p, c_longlong, c_int, c_int,
                        c_int, c_void_p]
     eg_gemm_tcgen05_pair = [c_void_p, c_int, c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_void_p, c_longlong, c_int, c_int,
@@ -528,7 +528,6 @@ SKINNY_MAX_TOKENS = int(os.environ.get("EASY_GPT_SKINNY_MAX_TOKENS", "16"))
 PREFETCH_WEIGHTS = os.environ.get("EASY_GPT_PREFETCH", "0") != "0"
 # every CTA repeats the norm prologue: worth it only for a few tokens (EASY_GPT_FUSED_NORM_MAX_TOKENS moves it)
 FUSED_NORM_MAX_TOKENS = int(os.environ.get("EASY_GPT_FUSED_NORM_MAX_TOKENS", "16"))
-WAIT_LIMIT = 1 << 22           # polls of a wait in gemm_stream.cu
 EPI_STORE, EPI_F32, EPI_SWIGLU, EPI_QKV_ROPE, EPI_RESID_NORM = 0, 1, 2, 3, 4
 # Programmatic dependent launch between the decode kernels (EASY_GPT_PDL).  2: a kernel lets the next one start when it has
 # passed its own wait (the next one then streams its first weights while this one works); 1: at its very start, so
@@ -618,7 +617,7 @@ def gemm_skinny(weight: torch.Tensor, bias: Optional[torch.Tensor], out: Optiona
                 gain: Optional[torch.Tensor] = None, eps: float = 0.0, tokens: Optional[int] = None,
                 plan=None, rope: Optional[dict] = None, prefetch: Optional[torch.Tensor] = None,
                 status: Optional[torch.Tensor] = None, prenormed: Optional[tuple] = None,
-                follow: Optional[dict] = None, norm=None, kernel: int = 0, wait_limit: Optional[int] = None):
+                follow: Optional[dict] = None, norm=None, kernel: int = 0, give_up: bool = False):
     """Decode-step product out = f(x W^T + bias) for up to 64 tokens, bfloat16 weights
     streamed once.  The input is ``x`` (bfloat16 [M, K]), or the norm prologue (``resid_in``,
     optional ``delta`` and ``resid_out``, ``gain``, ``eps``), or ``prenormed`` = (xn, ss_parts)
@@ -633,9 +632,9 @@ def gemm_skinny(weight: torch.Tensor, bias: Optional[torch.Tensor], out: Optiona
     same input given as one object with the fields eps, gain, residual, delta, residual_out,
     prepared_rows, prepared_sums (``parts.base.NormInFront``).  ``status``:
     the step's status word, where the bounded wait for the prologue's staged input reports
-    if it gives up.  ``kernel`` and ``wait_limit``, for tests and measurements: 1 or 2 for the kernel of
-    ``gemm_stream.cu`` (a KernelError where that does not take the sizes) or of ``gemm_skinny.cu``, and the
-    polls after which the former's waits give up."""
+    if it gives up.  ``kernel`` and ``give_up``, for tests and measurements: 1 or 2 for the kernel of
+    ``gemm_stream.cu`` (a KernelError where that does not take the sizes) or of ``gemm_skinny.cu``, and
+    whether the former's waits give up at once."""
     if norm is not None:
         eps = norm.eps
         if norm.prepared_rows is not None:
@@ -704,8 +703,8 @@ def gemm_skinny(weight: torch.Tensor, bias: Optional[torch.Tensor], out: Optiona
         groups = -(-N // (rb * 16))
         scratch, counters = _scratch_for(weight.device, split * groups * rb * 16 * skinny_padded_tokens(M), groups)
     launch = library().eg_gemm_skinny
-    if kernel or wait_limit is not None:
-        launch = functools.partial(library().eg_gemm_decode, kernel, WAIT_LIMIT if wait_limit is None else wait_limit)
+    if kernel or give_up:
+        launch = functools.partial(library().eg_gemm_decode, kernel, int(give_up))
     _check(launch(
         _stream(), epilogue, norm_mode, USE_PDL, _ptr(weight), weight.stride(0), _ptr(bias), M, N, K,
         _ptr(x), 0 if norm_mode else x.stride(0), _ptr(resid_in), _ptr(resid_out), _ptr(delta), _ptr(gain), float(eps),

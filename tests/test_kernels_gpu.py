@@ -703,7 +703,7 @@ def test_gemm_stream_units_splits_and_shares(M, N, K):
 @pytest.mark.parametrize("M", [1, 16])
 @pytest.mark.parametrize("N, K", [(48, 80), (896, 896), (896, 4864), (200, 2064), (6416, 2064), (19001, 896)])
 def test_gemm_stream_whose_waits_give_up_leaves_nothing_behind(M, N, K):
-    """Waits that give up at their first poll, while the weights are on their way: all stages asked for at once and a ring that
+    """Waits that give up at once, while the weights are on their way: all stages asked for at once and a ring that
     would go round, one CTA and clusters, one unit and shares.  The kernel says so and returns, and the next launches are right."""
     from easy_gpt.cpp_b200 import kernels
 
@@ -713,7 +713,7 @@ def test_gemm_stream_whose_waits_give_up_leaves_nothing_behind(M, N, K):
     kernels.gemm_skinny(w, None, before, kernels.EPI_F32, x=x, kernel=1, status=status)
     assert status.item() == 0
     for _ in range(20):
-        kernels.gemm_skinny(w, None, lost, kernels.EPI_F32, x=x, kernel=1, wait_limit=0, status=status)
+        kernels.gemm_skinny(w, None, lost, kernels.EPI_F32, x=x, kernel=1, give_up=True, status=status)
     kernels.gemm_skinny(w, None, after, kernels.EPI_F32, x=x, kernel=1)
     assert status.item() == 8
     assert torch.equal(before, after)
