@@ -102,16 +102,18 @@ __device__ __forceinline__ void store4(bf16* p, int q, float4 v) {
 }
 __device__ __forceinline__ float squares(float4 v) { return v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w; }
 
-// FEW: launches of few rows (a warp a block) keep the gain in registers too, read in front of the dependency wait
+// FEW: launches of few rows (a warp a block) keep the gain in registers too, asked for together with the row (behind the
+// dependency wait: a caller's stream may hold the kernel that writes it; the L2 is asked for it in front)
 template <typename TD, int VPL, bool FEW>
 __global__ void __launch_bounds__(FEW ? 32 : 256) rmsnorm_add_warp_kernel(float* __restrict__ stream, const TD* __restrict__ y, long long ldy,
                                                                           const float* __restrict__ gain, float eps, int tokens, int hidden) {
+    prefetch_weights(gain, hidden);
+    pdl_enter();
     float4 ahead[FEW ? VPL : 1];
     if (FEW)
 #pragma unroll
         for (int i = 0; i < VPL; ++i)
             if (i * 32 + (int)threadIdx.x < hidden / 4) ahead[i] = load4(gain, i * 32 + threadIdx.x);
-    pdl_enter();
     const int lane = threadIdx.x & 31;
     const int t = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (t >= tokens) return;
@@ -234,8 +236,8 @@ __global__ void __launch_bounds__(256) rmsnorm_add_norm_warp_kernel(float* __res
     }
 }
 
-// Few rows: a block per row, everything in registers and asked for at once (the weights in front of the dependency wait), both
-// rows' squares in one round through shared memory.  VPT float4 a thread.  (Measured on B200, 8 rows of 2,048 inside a decode
+// Few rows: a block per row, everything in registers and asked for at once, behind the dependency wait (nothing is read ahead of
+// the stream's order; the L2 is asked for the weights in front of it), both rows' squares in one round through shared memory.  VPT float4 a thread.  (Measured on B200, 8 rows of 2,048 inside a decode
 // step of six such layers: two passes over both rows with a round each, and the norm-and-add behind a branch reading its gain
 // last, took 462 us a step; with this kernel and the gain ahead 423.)
 template <typename TO, int VPT>
@@ -247,19 +249,21 @@ __global__ void __launch_bounds__(256) rmsnorm_shift_row_kernel(const float* __r
     const int quads = hidden / 4, t = blockIdx.x;
     const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
     float4 g[VPT], w[VPT], v[VPT], o[VPT], p[VPT];
+    prefetch_weights(gain, hidden);
+    prefetch_weights(mu, hidden);
+    pdl_enter();
+    const float* x = stream + (size_t)t * hidden;
+    const int seq = token_seq[t];
 #pragma unroll
     for (int i = 0; i < VPT; ++i) {
         const int q = i * 256 + threadIdx.x;
+        v[i] = q < quads ? load4(x, q) : zero;
         g[i] = q < quads ? load4(gain, q) : zero;
         w[i] = q < quads ? load4(mu, q) : zero;
     }
-    // (the batch's tables were there before the step began)
-    const int seq = token_seq[t];
     const bool first = t == seq_starts[seq];
     const int behind = seq_starts[seq + 1] - 1;
     float* slot = state + (size_t)seq_slots[seq] * slot_floats;
-    pdl_enter();
-    const float* x = stream + (size_t)t * hidden;
     // the row in front: the stream's row t-1 normed again here, or the slot's row; the first token's block also norms the
     // entry's last row for the slot
     const float* other = stream + (size_t)(first ? behind : t - 1) * hidden;
@@ -267,7 +271,6 @@ __global__ void __launch_bounds__(256) rmsnorm_shift_row_kernel(const float* __r
 #pragma unroll
     for (int i = 0; i < VPT; ++i) {
         const int q = i * 256 + threadIdx.x;
-        v[i] = q < quads ? load4(x, q) : zero;
         o[i] = q < quads ? load4(other, q) : zero;
         p[i] = first && q < quads ? load4(slot, q) : zero;
     }

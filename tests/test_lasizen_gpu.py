@@ -458,3 +458,45 @@ def test_norm_and_shift_of_few_rows(hidden, entries):
     # float32 sums of `hidden` squares and four roundings behind them
     assert float((out.cpu().double() - want).abs().max()) <= 2e-6 * float(want.abs().max())
     assert float((d[3].cpu().double() - want_state).abs().max()) <= 2e-6 * float(want_state.abs().max())
+
+
+def test_norms_read_gains_that_the_kernel_in_front_writes():
+    """A product writes the gain and the shift's weights, the norm behind it on the same stream uses them: the norms start early
+    (programmatic dependents) and still read them, and the batch's tables, in the stream's order."""
+    import ctypes
+
+    import torch
+
+    from easy_gpt.cpp_b200 import kernels
+
+    hidden, K, T = 2048, 32768, 4
+    g = torch.Generator().manual_seed(5)
+    w = (torch.randn(hidden, K, generator=g) * 0.01).bfloat16().cuda()
+    lib, P, F, I, LL = kernels.library(), ctypes.c_void_p, ctypes.c_float, ctypes.c_int, ctypes.c_longlong
+    at = lambda t: P(t.data_ptr())  # noqa: E731
+    for fn in (lib.eg_rmsnorm_add, lib.eg_rmsnorm_shift):
+        fn.restype = I
+    side = torch.cuda.Stream()
+    with torch.cuda.stream(side):
+        handle = P(side.cuda_stream)
+        for _ in range(5):
+            c = torch.randn(2, K, generator=g).bfloat16().cuda()
+            y, z, state = (torch.randn(T, hidden, generator=g).cuda() for _ in range(3))
+            gain = torch.zeros(2, hidden, device="cuda")
+            seq, starts = torch.arange(T, dtype=torch.int32, device="cuda"), torch.arange(T + 1, dtype=torch.int32, device="cuda")
+            out = torch.empty(T, hidden, device="cuda")
+            made = (c.double() @ w.double().t())
+            normed = y.double() / torch.sqrt((y.double() ** 2).mean(1, keepdim=True) + 1e-6) * made[0]
+            want_add, want_shift = z.double() + normed, normed + (state.double() - normed) * made[1]
+            torch.cuda.synchronize()
+            torch.cuda._sleep(400000)                              # the launches below queue up behind one another
+            kernels.gemm_skinny(w, None, gain, kernels.EPI_F32, x=c)
+            assert lib.eg_rmsnorm_add(handle, at(z), at(y), I(0), LL(hidden), at(gain), F(1e-6), I(T), I(hidden)) == 0
+            gain.zero_()
+            kernels.gemm_skinny(w, None, gain, kernels.EPI_F32, x=c)
+            assert lib.eg_rmsnorm_shift(handle, at(y), at(gain), F(1e-6), at(gain[1]), at(state), LL(hidden), at(seq), at(starts), at(seq), at(out), I(0),
+                                        I(T), I(hidden)) == 0
+            torch.cuda.synchronize()
+            # float32 sums of K = 32,768 products of order 0.01 behind them
+            assert float((z.double() - want_add).abs().max()) <= 1e-4 * float(want_add.abs().max())
+            assert float((out.double() - want_shift).abs().max()) <= 1e-4 * float(want_shift.abs().max())
