@@ -12,28 +12,28 @@
 //   products  mma.m16n8k16 with 16 weight rows as its M side and the tokens as its N side, both by ldmatrix; eight warps are
 //             row blocks x slices of K, a warp has one 64-term tile of every stage.
 //   sums      the slices meet in shared memory, CTAs that share a K range (a cluster) in the first one's: st.async counts
-//             on its mbarrier, the others are done at once.  Always in the same order, whatever the batch.
+//             on its mbarrier, the others are done at once.  Always in the same order, for 1 to 16 tokens (gemm_stream_plan.h
+//             decides by the epilogue, N and K alone which products are taken and how they are cut).
 //
 // Wide matrices: CTAs walk over consecutive row blocks, a unit at a time; the ring runs on across units.
 // Prologues and epilogues are those of gemm_skinny.cu (plain rows or prepared ones with partial sums of squares).
 // Every wait is bounded.
 #define EG_NEEDS_TENSOR_MAPS
 #include "gemm_skinny.cuh"
+#include "gemm_stream_plan.h"
 #include "mbarrier.cuh"
 #include "mma_utils.cuh"
 
 namespace {
 using namespace skinny;
+using stream_plan::MAX_STAGES;
+using stream_plan::MOST_SHARED;
+using stream_plan::RED_LD;
+using stream_plan::STAGE_BYTES;
+using stream_plan::WARPS;                     // that multiply; one more warp issues the copies
 
-constexpr int WARPS = 8;                      // that multiply; one more warp issues the copies
 constexpr int THREADS = (WARPS + 1) * 32;
-constexpr int MAX_STAGES = 16;
-constexpr int STAGE_BYTES = WARPS * 2048;     // a tile of 16 rows x 64 terms a warp
-constexpr int RED_LD = 20;                    // a token's 16 row sums: stores and loads of the warps' sums meet no bank twice
 constexpr int PREFETCH_PIECE = 16 * 1024;
-constexpr int SMS = 148;                       // a constant, so that results do not hang off the GPU
-constexpr int WIDE_BLOCKS = 400;              // row blocks from which on CTAs read all of K
-constexpr int MOST_SHARED = 220 * 1024;
 constexpr unsigned PARTS_WAIT_LIMIT = WAIT_LIMIT << 7;
 
 struct Plan {
@@ -448,64 +448,23 @@ namespace {
 template <int NT, int EPI, int NORM, bool GIVE_UP = false>
 int launch(cudaStream_t stream, const Params& p) {
     constexpr int MT = NT * 8;
+    constexpr bool pairs = EPI == EPI_QKV_ROPE, walks = !pairs && EPI != EPI_RESID_NORM;
+    stream_plan::Cut cut;
+    if (!stream_plan::cut_for(p.N, p.K, pairs, walks, &cut)) return -1;
+    const stream_plan::Ring ring = stream_plan::ring_of(cut, p.N, MT, walks);
+    const int rows = 16 << cut.rb_log, grid = ring.grid, split = cut.split;
     Plan s{};
+    s.rb_log = cut.rb_log;
+    s.stages = ring.stages;
+    s.k_len = cut.k_len;
+    s.k_stages = cut.k_stages;
     s.blocks = (p.N + 15) / 16;
-    int split = 1;
-    // How the CTAs share the matrix; from N and K alone, so that a sum's order does not hang off the batch.  (Measured on
-    // B200, us a decode step of 8 tokens at the 0.5B sizes / of 4 at the 1.5B sizes.)
-    if (EPI == EPI_QKV_ROPE) {
-        // a unit is 32 rows; its K is cut where that leaves a CTA 768 terms (0.5B, K 896: cut in two 591, whole 586; 1.5B,
-        // K 1536: 1,110 and 1,147)
-        s.rb_log = 1;
-        while (split < 8 && s.blocks * split <= SMS && p.K >= 768 * split * 2) split *= 2;
-    } else if (s.blocks >= WIDE_BLOCKS) {
-        s.rb_log = 2;                                             // (units of 128 rows: 620 / 1,155 against 623 / 1,078)
-    } else {
-        // As many CTAs as SMs: one each leaves room for the next kernel's (down product, 56 row blocks x 4,864: 112 CTAs 597,
-        // 224 CTAs 623).  Two an SM where one would have more than about 128 KB to read (1.5B: 96 CTAs 1,110, 192 CTAs 1,036).
-        // A CTA keeps 1,024 terms at least (K 896 cut in two: 575 against 562 for one token); of equal splits the one
-        // with the most rows a unit, since every CTA reads its range of x.  Powers of two: clusters of 5 and 6 do not all
-        // find room together.
-        const long long most = (long long)p.N * p.K * 2 > SMS * (128LL << 10) ? 2 * SMS : SMS;
-        long long best = -1;
-        for (int rb = 0; rb <= 2; ++rb) {
-            const int u = (s.blocks + (1 << rb) - 1) >> rb;
-            int cut = 1;
-            while (cut < 8 && (long long)u * cut * 2 <= most && p.K >= 1024 * cut * 2) cut *= 2;
-            const long long ctas = u * cut > most ? 2 * most - u * cut : u * cut;
-            if (ctas >= best && (rb == 0 || cut > 1)) {
-                best = ctas;
-                s.rb_log = rb;
-                split = cut;
-            }
-        }
-    }
-    const int RB = 1 << s.rb_log, KS = WARPS >> s.rb_log, rows = RB * 16;
-    const int units = EPI == EPI_QKV_ROPE ? s.blocks / 2 : (s.blocks + RB - 1) / RB;
-    s.k_len = ((p.K + split - 1) / split + 63) / 64 * 64;
-    split = (p.K + s.k_len - 1) / s.k_len;
-    s.k_stages = (s.k_len + KS * 64 - 1) / (KS * 64);
-    const int x_bytes = MT * (s.k_len * 2 + 16), red_bytes = WARPS * MT * RED_LD * 4, parts_bytes = split > 1 ? (split - 1) * rows * MT * 4 : 0;
-    const int rest = x_bytes + red_bytes + parts_bytes + 1024 + 64;
-    // two CTAs an SM (or this one and the next kernel's) unless x alone is more than half of that (16 tokens at the 1.5B sizes:
-    // 1,329 us a step with two, 1,463 with one)
-    const int budget = rest <= 80 * 1024 ? 110 * 1024 : MOST_SHARED;
-    const int per_sm = budget > 113 * 1024 ? 1 : 2;
-    int grid = units, stages_most = s.k_stages;
-    if (split == 1 && EPI != EPI_QKV_ROPE && EPI != EPI_RESID_NORM && grid > per_sm * SMS) {
-        grid = per_sm * SMS;
-        s.share = s.blocks / grid;
-        s.longer = s.blocks % grid;
-        stages_most = s.k_stages * ((s.share + RB) / RB);
-    }
-    s.stages = (budget - rest) / STAGE_BYTES;
-    if (s.stages > MAX_STAGES) s.stages = MAX_STAGES;
-    if (s.stages > stages_most) s.stages = stages_most;
-    if (s.stages < (stages_most > 1 ? 2 : 1)) return -1;
+    s.share = ring.share;
+    s.longer = ring.longer;
     s.x_offset = s.stages * STAGE_BYTES;
-    s.red_offset = (s.x_offset + x_bytes + 15) / 16 * 16;
-    s.parts_offset = (s.red_offset + red_bytes + 15) / 16 * 16;
-    const int smem = 1024 + s.parts_offset + parts_bytes;
+    s.red_offset = (s.x_offset + ring.x_bytes + 15) / 16 * 16;
+    s.parts_offset = (s.red_offset + ring.red_bytes + 15) / 16 * 16;
+    const int smem = 1024 + s.parts_offset + ring.parts_bytes;
     const eg_encode_tiled_fn encode = eg_encode_tiled();
     if (!encode) return -1;
     CUtensorMap maps[2];
@@ -532,14 +491,6 @@ int launch(cudaStream_t stream, const Params& p) {
         attr[n].val.clusterDim.y = (unsigned)split;
         attr[n].val.clusterDim.z = 1;
         ++n;
-        // all clusters have to find room together, or the last ones run as a second wave
-        cfg.attrs = attr;
-        cfg.numAttrs = n;
-        int clusters = 0;
-        if (cudaOccupancyMaxActiveClusters(&clusters, kernel, &cfg) != cudaSuccess || clusters < grid) {
-            (void)cudaGetLastError();
-            return -1;
-        }
     }
     if (p.use_pdl) {
         attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -580,4 +531,19 @@ int eg_gemm_stream_launch(cudaStream_t stream, int epilogue, int norm, const Par
     }
 #undef EG_STREAM_CASE
     return -1;
+}
+
+// The plan, for tests: out[0] whether the products of this epilogue and these sizes are taken (for 1 to 16 tokens alike), out[1..3] row
+// blocks a unit (log2), CTAs a unit's K is cut across, terms of each; for `tokens` tokens out[4..7] CTAs an SM, stages of the ring, CTAs or
+// clusters, row blocks of the shares (0: a unit each).
+EG_API int eg_gemm_stream_plan(int epilogue, int N, int K, int tokens, int* out) {
+    if (epilogue < 0 || epilogue > EPI_RESID_NORM || tokens < 1 || tokens > stream_plan::MOST_TOKENS || !out) return (int)cudaErrorInvalidValue;
+    const bool pairs = epilogue == EPI_QKV_ROPE, walks = !pairs && epilogue != EPI_RESID_NORM;
+    stream_plan::Cut c{};
+    out[0] = stream_plan::cut_for(N, K, pairs, walks, &c);
+    if (!out[0]) return 0;
+    const stream_plan::Ring r = stream_plan::ring_of(c, N, (tokens + 7) / 8 * 8, walks);
+    const int values[7] = {c.rb_log, c.split, c.k_len, r.per_sm, r.stages, r.grid, r.share};
+    for (int i = 0; i < 7; ++i) out[i + 1] = values[i];
+    return 0;
 }

@@ -85,6 +85,7 @@ class _Signatures:
                       c_longlong, c_longlong, c_void_p, c_void_p, c_longlong, c_void_p, c_void_p, c_int, c_void_p, c_void_p,
                       c_void_p, c_void_p]
     eg_gemm_decode = [c_int, c_int, *eg_gemm_skinny]
+    eg_gemm_stream_plan = [c_int, c_int, c_int, c_int, c_void_p]
     eg_gemm_tcgen05 = [c_void_p, c_int, c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_void_p, c_longlong, c_int, c_int,
                        c_int, c_void_p]
     eg_gemm_tcgen05_pair = [c_void_p, c_int, c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_void_p, c_longlong, c_int, c_int,
@@ -609,6 +610,14 @@ def _scratch_for(device, floats: int, row_groups: int):
 def skinny_padded_tokens(tokens: int) -> int:
     """The token tile of ``gemm_skinny`` for this many tokens (8, 16, 32 or 64)."""
     return 8 if tokens <= 8 else 16 if tokens <= 16 else 32 if tokens <= 32 else 64
+
+
+def gemm_stream_plan(epilogue: int, out_features: int, in_features: int, tokens: int):
+    """How ``csrc/gemm_stream.cu`` shares a product of up to 16 tokens out, None if it does not take it: (row blocks a unit (log2), CTAs a
+    unit's K is cut across, terms of each, CTAs an SM, stages of the ring, CTAs or clusters, row blocks of a share)."""
+    out = (c_int * 8)()
+    _check(library().eg_gemm_stream_plan(epilogue, out_features, in_features, tokens, out), "gemm_stream_plan")
+    return tuple(out[1:]) if out[0] else None
 
 
 def gemm_skinny(weight: torch.Tensor, bias: Optional[torch.Tensor], out: Optional[torch.Tensor], epilogue: int, *,

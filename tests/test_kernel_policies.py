@@ -57,3 +57,32 @@ def test_the_native_engine_plans_like_the_pytorch_face():
     for tiles in (1, 2, 3, 4, 8, 16, 40, 200):
         for heads, head in ((14, 64), (12, 128), (28, 128), (4, 64)):
             assert native.plan(3, tiles, heads, head, 2048)[:2] == tuple(kernels.attention_prefill_parts(tiles, heads, head)), (tiles, heads, head)
+
+
+def test_the_streaming_product_is_planned_alike_for_1_to_16_tokens():
+    """Which products the streaming kernel takes, and the order of their sums, hang off the epilogue, N and K alone; what a token tile
+    decides (the ring, CTAs an SM) has to fit: sizes of real models among them where a tile of 16 tokens fits and one of 8 does not, or
+    the other way round."""
+    sizes = [(n, k) for n in (8, 900, 896, 1536, 2048, 2560, 3072, 3584, 4096, 5120, 6416, 9728, 37888, 151936)
+             for k in (16, 208, 896, 1536, 2064, 4864, 8192, 8960, 11008, 13824, 14336, 18944)]
+    taken = 0
+    for epilogue in range(5):
+        for n, k in sizes:
+            if epilogue == kernels.EPI_QKV_ROPE and n % 32:
+                continue
+            plans = [kernels.gemm_stream_plan(epilogue, n, k, m) for m in range(1, 17)]
+            assert len({p[:3] if p else None for p in plans}) == 1, (epilogue, n, k, plans[0], plans[-1])
+            for m, p in enumerate(plans, 1):
+                if p is None:
+                    continue
+                taken += 1
+                rb_log, split, k_len, per_sm, stages, grid, share = p
+                tile, rows = 8 if m <= 8 else 16, 16 << rb_log
+                assert split in (1, 2, 3, 4, 5, 6, 7, 8) and (split - 1) * k_len < k <= split * k_len and k_len % 64 == 0
+                assert (grid * share if share else grid * (rows >> 4)) * 16 >= n - grid * 16
+                shared = 2048 + stages * 16384 + tile * (k_len * 2 + 16) + 8 * tile * 80 + (split - 1) * rows * tile * 4
+                assert 1 <= stages <= 16 and shared * per_sm <= 227 * 1024, (epilogue, n, k, m, p)
+                if split > 1:
+                    assert grid * split <= 148 * per_sm and not share
+    assert taken > 2000
+    assert kernels.gemm_stream_plan(kernels.EPI_F32, 2048, 11008, 16) and not kernels.gemm_stream_plan(kernels.EPI_F32, 5120, 13824, 1)

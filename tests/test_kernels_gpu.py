@@ -700,6 +700,22 @@ def test_gemm_stream_units_splits_and_shares(M, N, K):
     assert float((out.cpu() - want).abs().max()) <= 1e-5 * float(want.abs().max()) * math.sqrt(K)       # float32 accumulation
 
 
+@pytest.mark.parametrize("N, K", [(900, 896), (1536, 8960), (2048, 11008), (3072, 8192), (4096, 14336), (8192, 8192), (6416, 80)])
+def test_decode_product_of_a_row_does_not_hang_off_the_batch(N, K):
+    """Whichever kernel takes the sizes: the same bits for 1 to 16 tokens, among them sizes whose x fits shared memory in one token
+    tile and not in the other."""
+    from easy_gpt.cpp_b200 import kernels
+
+    x = bf(torch.randn(16, K, generator=gen(92))).to(DEV)
+    w = torch.empty(N, K, dtype=torch.bfloat16, device=DEV).normal_(0, 0.1)
+    whole = torch.empty(16, N, device=DEV)
+    kernels.gemm_skinny(w, None, whole, kernels.EPI_F32, x=x)
+    for M in (1, 7, 8, 9):
+        out = torch.empty(M, N, device=DEV)
+        kernels.gemm_skinny(w, None, out, kernels.EPI_F32, x=x[16 - M:])
+        assert torch.equal(out, whole[16 - M:]), M
+
+
 @pytest.mark.parametrize("M", [1, 16])
 @pytest.mark.parametrize("N, K", [(48, 80), (896, 896), (896, 4864), (200, 2064), (6416, 2064), (19001, 896)])
 def test_gemm_stream_whose_waits_give_up_leaves_nothing_behind(M, N, K):
