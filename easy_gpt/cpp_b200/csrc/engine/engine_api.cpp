@@ -300,7 +300,8 @@ EGE_API long long ege_runner_info(void* r, int what, int arg) {
 // what 0: the decode product's plan for (rows, width, head size or 0) -> (row blocks, K slices, K parts); 1: the decode
 // attention's splits for (tokens, heads, KV heads, longest context, head size); 2: the most tokens whose norm rides in
 // a decode product's prologue, for (width); 3: the prompt attention's (most parts, fewest key tiles of a part) for
-// (query tiles, heads, head size, longest context); 4: the SM count the plans hang off.
+// (query tiles, heads, head size, longest context); 4: the SM count the plans hang off; 5: how much of a first matrix of so many bytes is asked
+// for ahead.
 EGE_API void ege_plan(int what, const long long* in, long long* out) {
     switch (what) {
         case 0: {
@@ -320,5 +321,6 @@ EGE_API void ege_plan(int what, const long long* in, long long* out) {
             break;
         }
         case 4: out[0] = plans::sm_count(); break;
+        case 5: out[0] = (long long)plans::soon_bytes((size_t)in[0]); break;
     }
 }

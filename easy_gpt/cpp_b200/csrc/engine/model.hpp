@@ -240,6 +240,7 @@ public:
             const FeedForward* next_part = i + 1 < sublayers.size() ? sublayers[i + 1].feed_forward.get() : nullptr;
             ctx.soon_bytes = 0;
             ctx.soon = next_part ? next_part->first_weights(&ctx.soon_bytes) : nullptr;
+            ctx.soon_bytes = plans::soon_bytes(ctx.soon_bytes);
             if (sub.plain_pre_norm) {
                 const int fused_rows = plans::fused_norm_max_tokens(sub.norm->size());
                 PendingNorm pending(ctx, sub.norm.get(), s.residual, s.delta, s.spare, work, T, nullptr, 0, fused_rows);

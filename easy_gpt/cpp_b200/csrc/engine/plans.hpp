@@ -147,6 +147,16 @@ inline bool gemm_skinny_takes(DType dtype, int tokens, int in_features) {
 }
 inline int skinny_padded_tokens(int tokens) { return tokens <= 8 ? 8 : tokens <= 16 ? 16 : tokens <= 32 ? 32 : 64; }
 
+// How much of the feed-forward's first matrix the output projection in front of it asks the L2 for: what arrives while the
+// projection runs, and nothing of a matrix that the L2 (126 MB) does not hold, whose first part would be gone before it is read.
+// (us a decode step of 1 / 8 requests, nothing, all of it and up to 32 MB asked for: 0.5B sizes, 17 MB, 553 / 577, 544 / 563 and
+// 545 / 563; 14 layers of 1.5B, 55 MB, 532 / 573, 515 / 553 and 514 / 552; 8 of 3B, 90 MB, 485 / 515, 472 / 514 and 476 / 511; 6 of 7B,
+// 272 MB, 775 / 866, 827 / 924 and 779 / 873.)
+inline size_t soon_bytes(size_t weight_bytes) {
+    constexpr size_t most = 32u << 20, l2 = 126u << 20;
+    return weight_bytes > l2 ? 0 : std::min(weight_bytes, most);
+}
+
 // Products wide and tall enough for the persistent tcgen05 kernel on CTA pairs (one tile per SM at least).
 inline bool gemm_tcgen05_wide_takes(DType dtype, int tokens, int out_features, int in_features) {
     // (with fewer tiles the library product and a SwiGLU kernel are faster: a decode step at batch 64 takes 1.74 ms with

@@ -86,3 +86,10 @@ def test_the_streaming_product_is_planned_alike_for_1_to_16_tokens():
                     assert grid * split <= 148 * per_sm and not share
     assert taken > 2000
     assert kernels.gemm_stream_plan(kernels.EPI_F32, 2048, 11008, 16) and not kernels.gemm_stream_plan(kernels.EPI_F32, 5120, 13824, 1)
+
+
+def test_no_more_is_asked_ahead_of_the_l2_than_it_can_hold():
+    from easy_gpt.cpp_b200 import native
+
+    for bytes_, want in ((0, 0), (17 << 20, 17 << 20), (32 << 20, 32 << 20), (55 << 20, 32 << 20), (126 << 20, 32 << 20), (37888 * 3584 * 2, 0), (1 << 40, 0)):
+        assert native.plan(5, bytes_)[0] == want, bytes_
