@@ -54,7 +54,11 @@ inline Ring ring_of(const Cut& c, int N, int token_tile, bool walks) {
     const int rest = r.x_bytes + r.red_bytes + r.parts_bytes + 1024 + 64;
     // two CTAs an SM (or this one and the next kernel's) unless x alone is more than half of that (16 tokens at the 1.5B sizes:
     // 1,329 us a step with two, 1,463 with one)
-    for (r.per_sm = rest <= 80 * 1024 ? 2 : 1; r.per_sm >= 1; --r.per_sm) {
+    // ... and unless each CTA can have an SM of its own and a long walk that a ring of two or three stages would not cover (us a decode
+    // step of one and 8 requests, with two / with one: 8 layers of the 3B sizes, down product in 4 parts, 494 / 487 and 520 / 516; 6
+    // of 7B, QKV, 775 / 757 and 866 / 858)
+    const bool lone = c.units * c.split <= SMS && c.k_stages >= 12 && (HALF_SHARED - rest) / STAGE_BYTES < 4;
+    for (r.per_sm = rest <= 80 * 1024 && !lone ? 2 : 1; r.per_sm >= 1; --r.per_sm) {
         r.grid = c.units;
         r.share = r.longer = 0;
         int most = c.k_stages;
