@@ -10,6 +10,7 @@ from __future__ import annotations
 
 import collections
 import ctypes
+import os
 import threading
 import weakref
 from ctypes import POINTER, c_char_p, c_float, c_int, c_longlong, c_void_p
@@ -59,6 +60,7 @@ def library() -> ctypes.CDLL:
             "ege_runner_end": (None, [c_void_p, c_longlong]),
             "ege_runner_info": (c_longlong, [c_void_p, c_int, c_int]),
             "ege_host_alloc": (c_void_p, [c_longlong]),
+            "ege_host_pin": (c_int, [c_void_p]),
             "ege_host_free": (None, [c_void_p]),
             "ege_plan": (None, [c_int, c_void_p, c_void_p]),
         }
@@ -225,33 +227,41 @@ class NativeEngine:
 
 
 class _HostBlocks:
-    """Page-locked host memory for the logits that a runner hands out, taken again once the array (and every view of it) is
-    gone.  The copy from the device into fresh pageable memory was most of a decode step of several requests: 16 rows of
-    151,936 logits took 2.1 to 4 ms behind a step of 1.4 ms, into page-locked memory 0.2.  At most LIMIT bytes are held;
-    beyond that, and for arrays of less than GRAIN bytes (where the copy costs nothing), the caller uses plain memory."""
+    """Host memory for the logits that a runner hands out, taken again once the array (and every view of it) is gone: fresh
+    memory costs a step of several requests more than the step itself (its pages; 16 rows of 151,936 logits 3 ms).  A block that is taken
+    again is page-locked, so that the copy from the device runs at the link's rate (those 16 rows: 0.6 ms into memory that is there, 0.2
+    page-locked); a caller that keeps its arrays pays for no lock.  A free block of up to twice the size wanted will do.  At most LIMIT
+    bytes are held (in whole mappings of the library's); beyond that, for arrays of less than GRAIN bytes (where the copy costs
+    nothing) and of more than MOST (all logits of a long prompt, whose sizes hardly come twice), the caller uses plain memory."""
 
-    LIMIT, GRAIN = 512 << 20, 64 << 10
+    LIMIT, MOST, GRAIN = 512 << 20, 64 << 20, 64 << 10
 
     def __init__(self, lib):
         self._lib, self._lock, self._closed, self._held = lib, threading.Lock(), False, 0
+        self._process = os.getpid()
         self._free = {}                                          # size -> addresses
+        self._locked = set()                                     # addresses of blocks that have been taken again
         self._returned = collections.deque()                     # (address, size): finalizers may run anywhere, so they take no lock
 
     def array(self, rows: int, columns: int):
         """An uninitialised float32 array [rows, columns], or None."""
         size = -(-rows * columns * 4 // self.GRAIN) * self.GRAIN
-        if rows * columns * 4 < self.GRAIN:
+        if rows * columns * 4 < self.GRAIN or size > self.MOST:
             return None
         with self._lock:
             while self._returned:
                 at, n = self._returned.popleft()
                 self._free.setdefault(n, []).append(at)
-            if self._free.get(size):
-                address = self._free[size].pop()
+            fit = min((n for n, blocks in self._free.items() if blocks and size <= n <= 2 * size), default=None)
+            if fit is not None:
+                size, address = fit, self._free[fit].pop()
+                if address not in self._locked:
+                    self._locked.add(address)
+                    self._lib.ege_host_pin(address)
             else:
                 for n, blocks in self._free.items():             # blocks of other sizes make room
                     while blocks and self._held + size > self.LIMIT:
-                        self._lib.ege_host_free(blocks.pop())
+                        self._drop(blocks.pop())
                         self._held -= n
                 address = self._lib.ege_host_alloc(size) if self._held + size <= self.LIMIT else None
                 if not address:
@@ -260,6 +270,11 @@ class _HostBlocks:
         memory = (c_float * (rows * columns)).from_address(address)
         weakref.finalize(memory, self._give_back, address, size).atexit = False
         return np.frombuffer(memory, dtype=np.float32).reshape(rows, columns)
+
+    def _drop(self, address: int) -> None:
+        self._locked.discard(address)
+        if os.getpid() == self._process:                         # (a child of fork() leaves its copies to its end)
+            self._lib.ege_host_free(address)
 
     def _give_back(self, address: int, size: int) -> None:
         self._returned.append((address, size))
@@ -272,7 +287,7 @@ class _HostBlocks:
                 address, _ = self._returned.popleft()
             except IndexError:
                 return
-            self._lib.ege_host_free(address)
+            self._drop(address)
 
     def close(self) -> None:
         """Frees what is not handed out; the rest is freed as its arrays go."""
@@ -281,7 +296,7 @@ class _HostBlocks:
         with self._lock:
             for blocks in self._free.values():
                 while blocks:
-                    self._lib.ege_host_free(blocks.pop())
+                    self._drop(blocks.pop())
 
 
 class NativeStepRunner:
