@@ -684,20 +684,119 @@ def test_prompt_attention_with_either_number_of_softmax_groups(groups):
     assert " passed" in out.stdout
 
 
-# -- the decode product with its weights through shared memory (gemm_stream.cu) ------------------
+# -- the decode products' two kernels: weights through shared memory (gemm_stream.cu, 1) and register-fed (gemm_skinny.cu, 2) ------
 
-@pytest.mark.parametrize("M", [1, 7, 16])
+def sums_within(K):
+    """Of float32 sums of K exact products, of their largest: K / 16 sums behind one another, each off by 2^-23 of it at most, as a random
+    walk, four times over."""
+    return 2 ** -23 * math.sqrt(K)
+
+
+def assert_rounded_once(out, want, slack):
+    """bfloat16 values of float64 ones: half a step of the format (at most 2^-8 of a value) and what the float32 sums are off by."""
+    out, want = out.double().cpu(), want.double().cpu()
+    over = (out - want).abs() - (want.abs() * 2 ** -8 + slack)
+    assert float(over.max()) <= 0, (float(over.max()), float(want.abs().max()))
+
+
+@pytest.mark.parametrize("kernel", [1, 2])
 @pytest.mark.parametrize("N, K", [(8, 16), (900, 896), (200, 2064), (896, 4864), (1030, 8208), (6416, 80), (19001, 208)])
-def test_gemm_stream_units_splits_and_shares(M, N, K):
+def test_gemm_stream_and_skinny_units_splits_and_shares(N, K, kernel):
     """Less than a row block, ragged last units, K whole and cut across clusters (one of them with a short last part), and
-    matrices whose CTAs walk over shares that are no whole units."""
+    matrices whose CTAs walk over shares that are no whole units; a row's bits are the same whatever the number of tokens."""
     from easy_gpt.cpp_b200 import kernels
 
-    x, w, b = bf(torch.randn(M, K, generator=gen(70))), bf(torch.randn(N, K, generator=gen(71)) * 0.1), torch.randn(N, generator=gen(72))
-    want = x.float() @ w.float().t() + b
-    out = torch.full((M, N), float("nan"), device=DEV)
-    kernels.gemm_skinny(w.to(DEV), b.to(DEV), out, kernels.EPI_F32, x=x.to(DEV))
-    assert float((out.cpu() - want).abs().max()) <= 1e-5 * float(want.abs().max()) * math.sqrt(K)       # float32 accumulation
+    x, w, b = bf(torch.randn(16, K, generator=gen(70))), bf(torch.randn(N, K, generator=gen(71)) * 0.1), torch.randn(N, generator=gen(72))
+    want = x.double() @ w.double().t() + b.double()
+    whole = torch.full((16, N), float("nan"), device=DEV)
+    x, w, b = x.to(DEV), w.to(DEV), b.to(DEV)
+    kernels.gemm_skinny(w, b, whole, kernels.EPI_F32, x=x, kernel=kernel)
+    assert float((whole.cpu() - want).abs().max()) <= sums_within(K) * float(want.abs().max())
+    for M in (1, 7, 8, 9):
+        out = torch.full((M, N), float("nan"), device=DEV)
+        kernels.gemm_skinny(w, b, out, kernels.EPI_F32, x=x[16 - M:], kernel=kernel)
+        assert torch.equal(out, whole[16 - M:]), M
+
+
+@pytest.mark.parametrize("kernel", [1, 2])
+@pytest.mark.parametrize("M", [1, 8, 9, 16])
+@pytest.mark.parametrize("H, I, J", [(896, 4864, 4864), (208, 2064, 9600), (1040, 304, 72)])
+def test_gemm_stream_and_skinny_residual_norm_then_swiglu(M, H, I, J, kernel):
+    from easy_gpt.cpp_b200 import kernels
+
+    act, w = bf(torch.randn(16, I, generator=gen(73))), bf(torch.randn(H, I, generator=gen(74)) * 0.05)
+    gate_up = bf(torch.randn(2 * J, H, generator=gen(75)) * 0.05)
+    resid, gain = torch.randn(16, H, generator=gen(76)) * 2, 1 + 0.1 * torch.randn(H, generator=gen(77))
+
+    def both(first):                                               # the last tokens from `first` on
+        r = resid[first:].to(DEV)
+        rows, ss = kernels.gemm_skinny(w.to(DEV), None, None, kernels.EPI_RESID_NORM, x=act[first:].to(DEV), follow=dict(residual=r, gain=gain.to(DEV)),
+                                       kernel=kernel)
+        out = torch.empty(16 - first, J, dtype=torch.bfloat16, device=DEV)
+        kernels.gemm_skinny(gate_up.to(DEV), None, out, kernels.EPI_SWIGLU, prenormed=(rows, ss), eps=1e-5, kernel=kernel)
+        return r.cpu(), rows.cpu(), ss.cpu(), out.cpu()
+
+    v, rows, ss, out = both(16 - M)
+    y = act[16 - M:].double() @ w.double().t()
+    # the delta is rounded to bfloat16, then added in float32
+    assert_rounded_once(v.double() - resid[16 - M:].double(), y, sums_within(I) * float(y.abs().max()) + 2 ** -24 * float(v.abs().max()))
+    assert torch.equal(rows, bf(gain * v))
+    assert torch.allclose(ss.double().sum(0)[:M], (v.double() ** 2).sum(1), rtol=2 ** -23 * math.sqrt(H))
+    factor = 1 / torch.sqrt((v.double() ** 2).mean(1, keepdim=True) + 1e-5)
+    z = rows.double() @ gate_up.double().t() * factor
+    want = z[:, 1::2] * torch.nn.functional.silu(z[:, 0::2])
+    # gate and up off by their sums, the product's derivatives of order one times the other factor
+    assert_rounded_once(out, want, 4 * sums_within(H) * float(z.abs().max()) ** 2)
+    if M < 16:
+        for mine, whole in zip((v, rows, out), (both(0)[i] for i in (0, 1, 3))):
+            assert torch.equal(mine, whole[16 - M:])
+
+
+@pytest.mark.parametrize("kernel", [1, 2])
+@pytest.mark.parametrize("M, NH, NKV, HD, K", [(1, 14, 2, 64, 896), (16, 3, 1, 96, 1616), (5, 12, 2, 128, 1536), (3, 2, 2, 32, 64), (7, 3, 1, 80, 640),
+                                               (9, 3, 1, 80, 640)])
+def test_gemm_stream_and_skinny_qkv_rope_cache(M, NH, NKV, HD, K, kernel):
+    """Pairs of row blocks per head, K whole and cut in two, a head of three pairs, and heads that only the register-fed kernel
+    takes: against product, rotation and cache rows."""
+    from easy_gpt.cpp_b200 import kernels
+    from easy_gpt.cpp_b200.parts.rope import RotaryEncoding
+
+    ps, pages, N = 16, 9, (NH + 2 * NKV) * HD
+    w, bias = bf(torch.randn(N, K, generator=gen(80)) * 0.05), torch.randn(N, generator=gen(81)) * 0.3
+    rows, ss = bf(torch.randn(M, K, generator=gen(82))), torch.zeros(3, kernels.skinny_padded_tokens(M))
+    ss[:, :M] = torch.rand(3, M, generator=gen(83)) * K
+    positions = torch.randint(0, 5000, (M,), generator=gen(84), dtype=torch.int32)
+    slots = torch.randperm(ps * pages, generator=gen(85))[:M].to(torch.int32)
+    inv, status = RotaryEncoding.inverse_frequencies(HD, 1e6), torch.zeros(1, dtype=torch.int32, device=DEV)
+    kc = torch.zeros(pages, NKV, ps, HD, dtype=torch.bfloat16, device=DEV)
+    vc, q = torch.zeros_like(kc), torch.empty(M, NH * HD, dtype=torch.bfloat16, device=DEV)
+
+    def launch():
+        kernels.gemm_skinny(w.to(DEV), bias.to(DEV), q, kernels.EPI_QKV_ROPE, prenormed=(rows.to(DEV), ss.to(DEV)), eps=1e-6, kernel=kernel,
+                            rope=dict(num_heads=NH, num_kv_heads=NKV, head_dim=HD, positions=positions.to(DEV), slot_map=slots.to(DEV), k_cache=kc,
+                                      v_cache=vc, inv_freq=inv.to(DEV), status=status))
+
+    if kernel == 1 and HD % 32:
+        with pytest.raises(kernels.KernelError):
+            launch()
+        return
+    launch()
+    assert status.item() == 0
+    full = rows.double() @ w.double().t() / torch.sqrt(ss.double().sum(0)[:M, None] / K + 1e-6) + bias
+    angle = (positions[:, None].float() * inv.float().cpu()).double()[:, None]                     # float32 angles, as the kernels and the plain model take them
+
+    def turned(h):
+        a, c = h[..., :HD // 2], h[..., HD // 2:]
+        return torch.cat([a * angle.cos() - c * angle.sin(), c * angle.cos() + a * angle.sin()], -1)
+
+    qw, kw = turned(full[:, :NH * HD].reshape(M, NH, HD)).reshape(M, -1), turned(full[:, NH * HD:(NH + NKV) * HD].reshape(M, NKV, HD))
+    vw = full[:, (NH + NKV) * HD:].reshape(M, NKV, HD)
+    slack = 4 * sums_within(K) * float(full.abs().max())
+    at = (slots.long() // ps, slice(None), slots.long() % ps)
+    assert_rounded_once(q, qw, slack)
+    assert_rounded_once(kc.cpu()[at], kw, slack)
+    assert_rounded_once(vc.cpu()[at], vw, slack)
+    assert int((kc.float().abs().sum(dim=(1, 3)) > 0).sum()) == M
 
 
 @pytest.mark.parametrize("N, K", [(900, 896), (1536, 8960), (2048, 11008), (3072, 8192), (4096, 14336), (8192, 8192), (6416, 80)])
@@ -733,59 +832,6 @@ def test_gemm_stream_whose_waits_give_up_leaves_nothing_behind(M, N, K):
     kernels.gemm_skinny(w, None, after, kernels.EPI_F32, x=x, kernel=1)
     assert status.item() == 8
     assert torch.equal(before, after)
-
-
-@pytest.mark.parametrize("M, H, I, J", [(1, 896, 4864, 4864), (16, 208, 2064, 9600), (9, 1040, 304, 72)])
-def test_gemm_stream_residual_norm_then_swiglu(M, H, I, J):
-    from easy_gpt.cpp_b200 import kernels
-
-    act, w = bf(torch.randn(M, I, generator=gen(73))), bf(torch.randn(H, I, generator=gen(74)) * 0.05)
-    gate_up = bf(torch.randn(2 * J, H, generator=gen(75)) * 0.05)
-    resid, gain = torch.randn(M, H, generator=gen(76)) * 2, 1 + 0.1 * torch.randn(H, generator=gen(77))
-    delta = bf(act.float() @ w.float().t()).float()
-    r = resid.to(DEV)
-    rows, ss = kernels.gemm_skinny(w.to(DEV), None, None, kernels.EPI_RESID_NORM, x=act.to(DEV), follow=dict(residual=r, gain=gain.to(DEV)))
-    v = r.cpu()
-    assert float((v - resid - delta).abs().max()) <= 2 ** -7 * float(delta.abs().max()) + 1e-6             # the delta is rounded to bfloat16
-    assert torch.equal(rows.cpu(), bf(gain * v))
-    assert torch.allclose(ss.sum(0).cpu()[:M], (v * v).sum(1), rtol=1e-5)
-    out = torch.empty(M, J, dtype=torch.bfloat16, device=DEV)
-    kernels.gemm_skinny(gate_up.to(DEV), None, out, kernels.EPI_SWIGLU, prenormed=(rows, ss), eps=1e-5)
-    factor = 1 / torch.sqrt((v * v).mean(1, keepdim=True) + 1e-5)
-    y = rows.float().cpu() @ gate_up.float().t() * factor
-    want = y[:, 1::2] * torch.nn.functional.silu(y[:, 0::2])
-    assert float((out.float().cpu() - want).abs().max()) <= 2 ** -7 * float(want.abs().max())              # rounded to bfloat16
-
-
-@pytest.mark.parametrize("M, NH, NKV, HD, K", [(1, 14, 2, 64, 896), (16, 3, 1, 96, 1616), (5, 12, 2, 128, 1536), (3, 2, 2, 32, 64)])
-def test_gemm_stream_qkv_rope_cache(M, NH, NKV, HD, K):
-    """Pairs of row blocks per head, K whole and cut in two, a head of three pairs: against product, rotation and cache rows."""
-    from easy_gpt.cpp_b200 import kernels
-    from easy_gpt.cpp_b200.parts.rope import RotaryEncoding
-
-    ps, pages, N = 16, 9, (NH + 2 * NKV) * HD
-    w, bias = bf(torch.randn(N, K, generator=gen(80)) * 0.05), torch.randn(N, generator=gen(81)) * 0.3
-    rows, ss = bf(torch.randn(M, K, generator=gen(82))), torch.zeros(3, kernels.skinny_padded_tokens(M))
-    ss[:, :M] = torch.rand(3, M, generator=gen(83)) * K
-    positions = torch.randint(0, 5000, (M,), generator=gen(84), dtype=torch.int32)
-    slots = torch.randperm(ps * pages, generator=gen(85))[:M].to(torch.int32)
-    inv, status = RotaryEncoding.inverse_frequencies(HD, 1e6), torch.zeros(1, dtype=torch.int32, device=DEV)
-    kc = torch.zeros(pages, NKV, ps, HD, dtype=torch.bfloat16, device=DEV)
-    vc, q = torch.zeros_like(kc), torch.empty(M, NH * HD, dtype=torch.bfloat16, device=DEV)
-    kernels.gemm_skinny(w.to(DEV), bias.to(DEV), q, kernels.EPI_QKV_ROPE, prenormed=(rows.to(DEV), ss.to(DEV)), eps=1e-6,
-                        rope=dict(num_heads=NH, num_kv_heads=NKV, head_dim=HD, positions=positions.to(DEV), slot_map=slots.to(DEV), k_cache=kc,
-                                  v_cache=vc, inv_freq=inv.to(DEV), status=status))
-    assert status.item() == 0
-    full = rows.float() @ w.float().t() / torch.sqrt(ss.sum(0)[:M, None] / K + 1e-6) + bias
-    qw = plain_model.rope(full[:, :NH * HD].reshape(M, NH, HD), positions.long(), 1e6).reshape(M, -1)
-    kw = plain_model.rope(full[:, NH * HD:(NH + NKV) * HD].reshape(M, NKV, HD), positions.long(), 1e6)
-    vw = full[:, (NH + NKV) * HD:].reshape(M, NKV, HD)
-    tol = 2 ** -7 * float(full.abs().max())                                                                 # rounded to bfloat16
-    assert float((q.float().cpu() - qw).abs().max()) <= tol
-    at = (slots.long() // ps, slice(None), slots.long() % ps)
-    assert float((kc.float().cpu()[at] - kw).abs().max()) <= tol
-    assert float((vc.float().cpu()[at] - vw).abs().max()) <= tol
-    assert int((kc.float().abs().sum(dim=(1, 3)) > 0).sum()) == M
 
 
 @pytest.mark.parametrize("NH, NKV, HD, ps, contexts, queries, window", [
