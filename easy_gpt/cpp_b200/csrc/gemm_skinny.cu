@@ -554,6 +554,14 @@ __global__ void __launch_bounds__(MAX_THREADS) skinny_kernel(const Params p) {
     }
 }
 
+// Prepared rows as this file's kernel stages them: aligned, in copies that one barrier counts, and within its shared memory.
+// (gemm_stream.cu could do with less, but what is taken does not hang off the kernel that happens to run.)
+bool takes_prepared_rows(const Params& p) {
+    const size_t tile = p.M <= 8 ? 8 : p.M <= 16 ? 16 : p.M <= 32 ? 32 : 64, K = (size_t)p.K, parts_bytes = (size_t)p.ss_parts * tile * sizeof(float);
+    const size_t rows_bytes = tile * ((K * 2 + 127) / 128 * 128 + 64) + tile * sizeof(float) + K * sizeof(float) + tile * 8 * sizeof(float);
+    return (uintptr_t)p.delta % 16 == 0 && (uintptr_t)p.ss_in % 16 == 0 && (size_t)p.M * K * 2 + parts_bytes < (1u << 20) && rows_bytes + parts_bytes <= 200 * 1024;
+}
+
 template <int NT, int EPI, int NORM>
 int launch_one(cudaStream_t stream, const Params& p_in, int ctas, int k_split) {
     constexpr int MT = NT * 8;
@@ -568,12 +576,7 @@ int launch_one(cudaStream_t stream, const Params& p_in, int ctas, int k_split) {
     size_t xs_bytes = NORM ? (size_t)MT * (((p.K * 2 + 127) / 128) * 128 + 64) + MT * sizeof(float) + (size_t)p.K * sizeof(float) + (size_t)MT * 8 * sizeof(float) : 0;
     // the residual rows staged in shared memory, where they fit and the copies' alignment rule (16 bytes) holds
     const size_t staged_bytes = (size_t)p.M * p.K * sizeof(float);
-    if (NORM == 2) {
-        const size_t parts_bytes = (size_t)p.ss_parts * MT * sizeof(float);
-        if ((uintptr_t)p.delta % 16 || (uintptr_t)p.ss_in % 16 || (size_t)p.M * p.K * 2 + parts_bytes >= (1u << 20))
-            return (int)cudaErrorInvalidValue;
-        xs_bytes += parts_bytes;
-    }
+    if (NORM == 2) xs_bytes += (size_t)p.ss_parts * MT * sizeof(float);
     p.stage_norm = NORM == 1 && xs_bytes + staged_bytes + (p.cluster_reduce ? parts_bytes_cluster + 16 : 0) <= 200 * 1024 && (uintptr_t)p.resid_in % 16 == 0 && (uintptr_t)p.delta % 16 == 0 &&
                    (size_t)p.M * p.K * 6 < (1u << 20);
     if (p.stage_norm) xs_bytes += staged_bytes;
@@ -680,6 +683,7 @@ static int gemm_skinny_any(cudaStream_t stream, int epilogue, int norm, int use_
     p.resid_inout = resid_inout; p.gain_out = gain_out; p.xn_out = (bf16*)xn_out; p.ss_out = ss_out;
     p.act = act; p.act_a = act_a; p.act_b = act_b;
     p.give_up = give_up;
+    if (norm == 2 && !takes_prepared_rows(p)) return (int)cudaErrorInvalidValue;
     const int taken = kernel == 2 ? -1 : eg_gemm_stream_launch(stream, epilogue, norm, p);
     if (taken >= 0) return taken;
     if (kernel == 1) return (int)cudaErrorInvalidValue;

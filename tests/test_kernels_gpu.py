@@ -799,6 +799,22 @@ def test_gemm_stream_and_skinny_qkv_rope_cache(M, NH, NKV, HD, K, kernel):
     assert int((kc.float().abs().sum(dim=(1, 3)) > 0).sum()) == M
 
 
+@pytest.mark.parametrize("kernel", [0, 1, 2])
+def test_prepared_rows_are_refused_alike_whichever_kernel_would_run(kernel):
+    """More than the register-fed kernel's shared memory holds, and partial sums that its bulk copy cannot start at."""
+    from easy_gpt.cpp_b200 import kernels
+
+    out = torch.empty(16, 640, device=DEV)
+    for K, offset, fits in ((8192, 0, False), (640, 1, False), (640, 0, True)):
+        w, rows = torch.zeros(640, K, dtype=torch.bfloat16, device=DEV), torch.zeros(16, K, dtype=torch.bfloat16, device=DEV)
+        sums = torch.ones(65, device=DEV)[offset:offset + 64].view(4, 16)
+        if fits:
+            kernels.gemm_skinny(w, None, out, kernels.EPI_F32, prenormed=(rows, sums), eps=1e-6, kernel=kernel)
+        else:
+            with pytest.raises(kernels.KernelError):
+                kernels.gemm_skinny(w, None, out, kernels.EPI_F32, prenormed=(rows, sums), eps=1e-6, kernel=kernel)
+
+
 @pytest.mark.parametrize("N, K", [(900, 896), (1536, 8960), (2048, 11008), (3072, 8192), (4096, 14336), (8192, 8192), (6416, 80)])
 def test_decode_product_of_a_row_does_not_hang_off_the_batch(N, K):
     """Whichever kernel takes the sizes: the same bits for 1 to 16 tokens, among them sizes whose x fits shared memory in one token
