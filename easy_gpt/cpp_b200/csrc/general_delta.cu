@@ -30,6 +30,8 @@
 // differ; two columns and P = 8, 445; with the outputs of four tokens summed over the lanes together, so that the loads of a token
 // do not wait for the stores of the token before, 345; one column a thread, so twice the warps, 302.)
 //
+// (Prompts through heads of 64 go in chunks of 16 tokens: general_delta_chunks.cuh.)
+//
 // Tiles arrive three stages ahead.  Outputs are normed and gated by the block where it holds a whole head, else by a kernel behind.
 // The slot keeps S as [head, column, row].  The order of every sum depends on the sizes and on a token's place in its block.
 #include <algorithm>
@@ -628,6 +630,27 @@ int dispatch_general_delta(cudaStream_t stream, const DeltaParams& p, int slices
     return launch_general_delta<TO, 8, 32, 2, INLINE>(stream, p, slices, num_seqs, wide);
 }
 
+#include "general_delta_chunks.cuh"
+
+// Which prompts go through the chain of chunks: heads of 64, entries of 32 tokens on average.
+bool chunks_take(int tokens, int num_seqs, int dim) { return dim == CHUNK_DIM && tokens >= 2 * CHUNK * num_seqs; }
+
+template <typename TO>
+int launch_chunks(cudaStream_t stream, DeltaParams p, int num_seqs, bool wide) {
+    constexpr int smem = CHUNK_STAGES * CHUNK_STAGE * 4;
+    static const cudaError_t configured = cudaFuncSetAttribute(general_delta_chain_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (configured != cudaSuccess) return (int)configured;
+    const int most_chunks = p.tokens / CHUNK + num_seqs;
+    const unsigned blocks = (unsigned)((long long)most_chunks * p.heads);
+    if (wide) eg_pdl_launch(general_delta_chunks_kernel<true>, blocks, 128, 0, stream, p, num_seqs, most_chunks);
+    else eg_pdl_launch(general_delta_chunks_kernel<false>, blocks, 128, 0, stream, p, num_seqs, most_chunks);
+    eg_pdl_launch_if(false, general_delta_chain_kernel, dim3(p.heads, num_seqs, CHUNK_DIM / CHUNK_COLS), 256, smem, stream, p, most_chunks);
+    p.lanes = CHUNK_DIM / 4;
+    if (wide) eg_pdl_launch(general_delta_output_kernel<TO, true>, (unsigned)(((long long)p.tokens * p.heads * p.lanes + 255) / 256), 256, 0, stream, p);
+    else eg_pdl_launch(general_delta_output_kernel<TO, false>, (unsigned)(((long long)p.tokens * p.heads + 7) / 8), 256, 0, stream, p);
+    return eg_launch_status();
+}
+
 template <typename T>
 __global__ void tanh_columns_kernel(const float* __restrict__ src, long long lds, T* __restrict__ dst, long long ldd, int rows, int cols, int padded) {
     pdl_enter();
@@ -638,8 +661,12 @@ __global__ void tanh_columns_kernel(const float* __restrict__ src, long long lds
 }
 }  // namespace
 
-// float32 values of a record of a head of `dim` channels (scratch: heads * tokens of them)
-EG_API int eg_general_delta_record(int dim) { return VECS * (dim <= 16 ? 16 : dim <= 32 ? 32 : dim <= 64 ? 64 : dim <= 128 ? 128 : 256) + NUMBERS; }
+// float32 values of scratch memory (`records`) a token and head of `dim` channels: a record, or a token's share of the chunks, of which
+// there are at most tokens / 16 + num_seqs <= 3 tokens / 32
+EG_API int eg_general_delta_record(int dim) {
+    if (dim == CHUNK_DIM) return std::max(VECS * 64 + NUMBERS, (3 * CHUNK_RECORD / 32 + 3) / 4 * 4);
+    return VECS * (dim <= 16 ? 16 : dim <= 32 ? 32 : dim <= 64 ? 64 : dim <= 128 ? 128 : 256) + NUMBERS;
+}
 
 // up to how many tokens an entry may have, and how large the inner size may be, for eg_general_delta with x null
 EG_API int eg_general_delta_inline_takes(int entry_tokens, int rank) { return entry_tokens <= 8 && rank <= 512; }
@@ -696,6 +723,8 @@ EG_API int eg_general_delta(cudaStream_t stream, const float* proj, long long ld
     auto aligned = [](const void* q) { return (uintptr_t)q % 16 == 0; };
     const bool wide = ldp % 4 == 0 && ldx % 4 == 0 && r_col % 4 == 0 && k_col % 4 == 0 && v_col % 4 == 0 && g_col % 4 == 0 && a_col % 4 == 0 && aligned(proj) &&
                       aligned(x) && aligned(w0) && aligned(a0) && aligned(gain) && aligned(o_raw) && aligned(y) && ldy % 4 == 0;
+    if (x && o_raw && (uintptr_t)o_raw % 8 == 0 && chunks_take(tokens, num_seqs, dim))
+        return y_dtype == EG_BF16 ? launch_chunks<bf16>(stream, p, num_seqs, wide) : launch_chunks<float>(stream, p, num_seqs, wide);
     if (y_dtype == EG_BF16)
         return x ? dispatch_general_delta<bf16, false>(stream, p, slices, num_seqs, wide) : dispatch_general_delta<bf16, true>(stream, p, slices, num_seqs, wide);
     return x ? dispatch_general_delta<float, false>(stream, p, slices, num_seqs, wide) : dispatch_general_delta<float, true>(stream, p, slices, num_seqs, wide);
