@@ -43,7 +43,8 @@ struct Layout {
     // up to five tiles in flight per CTA, within about 96 KB of shared memory (two stages at least)
     static constexpr int DEEP_STAGES = (TPI * 96 * 1024 / STAGE_BYTES) >= 5 ? 5 : ((TPI * 96 * 1024 / STAGE_BYTES) >= 2 ? (TPI * 96 * 1024 / STAGE_BYTES) : 2);
     static constexpr int STAGES = DEEP ? DEEP_STAGES : (DEEP_STAGES < 3 ? DEEP_STAGES : 3);
-    static constexpr int WARP_MERGE_BYTES = TPI * 4 * 16 * (HD + 2) * 4;      // the warps' partial results
+    static constexpr int MERGE_LD = HD + 8;                                   // floats of a row: eight rows' pairs meet no bank twice
+    static constexpr int WARP_MERGE_BYTES = TPI * 4 * 16 * (MERGE_LD + 2) * 4;      // the warps' partial results
     static constexpr int SPLIT_MERGE_BYTES = (2 * 16 * MAX_SPLITS + 16) * 4;  // (m, l) of every row and split, 1/l per row
     static constexpr int MERGE_BYTES = WARP_MERGE_BYTES > SPLIT_MERGE_BYTES ? WARP_MERGE_BYTES : SPLIT_MERGE_BYTES;
     static constexpr int SMEM = (STAGES * STAGE_BYTES > MERGE_BYTES) ? STAGES * STAGE_BYTES : MERGE_BYTES;
@@ -66,7 +67,7 @@ struct Params {
     long long page_stride, head_stride;
     const int* block_table;
     int table_stride;
-    const int* token_seq;
+    const int* token_seq;     // null: token i is sequence i's
     const int* positions;
     const int* seq_context;   // [sequences] keys cached before this step (those from it on are written by the kernel in front); may be null
     bf16* out;
@@ -152,11 +153,15 @@ __global__ void __launch_bounds__(TPI * THREADS) attention_paged_kernel(const Pa
     // Positions and block tables were uploaded before the step and the cached keys were written by earlier
     // steps, so everything up to the first fresh key can be fetched before the kernel in front has finished.
     if (p.use_pdl == 1) asm volatile("griddepcontrol.launch_dependents;\n" ::);
+    const int seq = p.token_seq ? p.token_seq[t] : t;
+    const int* table = p.block_table + (size_t)seq * p.table_stride;
+    // A run that begins with the first key: this thread's entry of the block table is asked for beside the position, not behind it
+    const bool from_start = p.splits == 1 && p.window <= 0 && x_chunk == 0;
+    const int early_page = from_start ? table[min((int)threadIdx.x * 16 / p.page_size, p.table_stride - 1)] : 0;
     const int pos = p.positions[t];
-    const int fresh_from = p.seq_context ? p.seq_context[p.token_seq[t]] : 0;
+    const int fresh_from = p.seq_context ? p.seq_context[seq] : 0;
     int first = (p.window > 0 && pos - p.window + 1 > 0) ? pos - p.window + 1 : 0;
     if (x_chunk > 0) first = max(first, pos / x_chunk * x_chunk);
-    const int* table = p.block_table + (size_t)p.token_seq[t] * p.table_stride;
     const int tile_lo = first / TILE_KEYS, tile_hi = pos / TILE_KEYS;           // inclusive
     // Key tiles in the order they are walked: those of the kept first keys that lie wholly in front of the others, then the
     // tiles from the first visible key on.  my_lo, my_hi and every tile index below count in that order; tile_of gives the tile.
@@ -180,7 +185,7 @@ __global__ void __launch_bounds__(TPI * THREADS) attention_paged_kernel(const Pa
             const int kpos0 = tile_of(tile0 + e / 4) * TILE_KEYS + (e % 4) * 16;
             long long base = -1;
             if (kpos0 <= pos && (kpos0 + 15 >= first || kpos0 < x_keep)) {
-                const int page = table[kpos0 / p.page_size];
+                const int page = from_start && tile0 == 0 && e == (int)threadIdx.x ? early_page : table[kpos0 / p.page_size];
                 if (page < 0 || page >= p.num_pages) atomicOr(p.status, EG_STATUS_BAD_PAGE);
                 else base = (long long)page * p.page_stride + (long long)kvh * p.head_stride + (long long)(kpos0 % p.page_size) * HD;
             }
@@ -361,7 +366,8 @@ __global__ void __launch_bounds__(TPI * THREADS) attention_paged_kernel(const Pa
     l1 += __shfl_xor_sync(0xffffffffu, l1, 2);
     float* wm = reinterpret_cast<float*>(smem);                                   // [WARPS][16]
     float* wl = wm + WARPS * 16;                                                  // [WARPS][16]
-    float* wacc = wl + WARPS * 16;                                                // [WARPS][16][HD]
+    float* wacc = wl + WARPS * 16;                                                // [WARPS][16][MERGE_LD]; rows of query heads only
+    const int rows = min(16, G - g0);
     if (tig == 0) {
         wm[warp * 16 + gid] = m0;
         wm[warp * 16 + gid + 8] = m1;
@@ -370,13 +376,9 @@ __global__ void __launch_bounds__(TPI * THREADS) attention_paged_kernel(const Pa
     }
 #pragma unroll
     for (int i = 0; i < HD / 8; ++i) {
-        const int d = i * 8 + 2 * tig;
-        float* a0 = wacc + ((warp * 16 + gid) * HD + d);
-        float* a1 = wacc + ((warp * 16 + gid + 8) * HD + d);
-        a0[0] = acc[i][0];
-        a0[1] = acc[i][1];
-        a1[0] = acc[i][2];
-        a1[1] = acc[i][3];
+        float* a0 = wacc + (warp * 16 + gid) * L::MERGE_LD + i * 8 + 2 * tig;
+        if (gid < rows) *reinterpret_cast<float2*>(a0) = make_float2(acc[i][0], acc[i][1]);
+        if (gid + 8 < rows) *reinterpret_cast<float2*>(a0 + 8 * L::MERGE_LD) = make_float2(acc[i][2], acc[i][3]);
     }
     // Splits as a cluster: every CTA of it is past its key tiles here, so the first CTA's pipeline memory is free for
     // the others' results (behind the part that its own warps' merge still uses).
@@ -390,42 +392,46 @@ __global__ void __launch_bounds__(TPI * THREADS) attention_paged_kernel(const Pa
     } else {
         __syncthreads();
     }
-    const int rows = min(16, G - g0);
-    for (int e = threadIdx.x; e < rows * HD; e += NT) {
-        const int r = e / HD, d = e % HD;
+    for (int e = threadIdx.x; e < rows * (HD / 2); e += NT) {
+        const int r = e / (HD / 2), d = e % (HD / 2) * 2;
         float m = -INFINITY;
 #pragma unroll
         for (int w = 0; w < WARPS; ++w) m = fmaxf(m, wm[w * 16 + r]);
-        float l = 0.f, a = 0.f;
+        float l = 0.f, a = 0.f, b = 0.f;
         if (m > -INFINITY) {
 #pragma unroll
             for (int w = 0; w < WARPS; ++w) {
                 const float f = exp2f(wm[w * 16 + r] - m);                          // -inf -> 0
+                const float2 v = *reinterpret_cast<const float2*>(wacc + (w * 16 + r) * L::MERGE_LD + d);
                 l += wl[w * 16 + r] * f;
-                a += wacc[(w * 16 + r) * HD + d] * f;
+                a += v.x * f;
+                b += v.y * f;
             }
         }
         const int h = kvh * G + g0 + r;
         if (p.splits == 1) {
             const float s2 = sink_of(g0 + r);
-            const float v = (s2 == -INFINITY ? (l > 0.f ? a / l : 0.f) : a * norm_with_sink(m, l, s2)) * x_out_scale;
+            const float norm = norm_with_sink(m, l, s2);
+            const float v0 = (s2 == -INFINITY ? (l > 0.f ? a / l : 0.f) : a * norm) * x_out_scale;
+            const float v1 = (s2 == -INFINITY ? (l > 0.f ? b / l : 0.f) : b * norm) * x_out_scale;
             const size_t at = (size_t)t * p.ldo + (size_t)head_of(g0 + r) * HD + d;
-            if (x_out_f32) x_out_f32[at] = v;
-            else p.out[at] = __float2bfloat16_rn(v);
+            if (x_out_f32) {
+                x_out_f32[at] = v0;
+                x_out_f32[at + 1] = v1;
+            } else if (p.ldo % 2 == 0 && (uintptr_t)p.out % 4 == 0) {
+                *reinterpret_cast<uint32_t*>(p.out + at) = pack_bf16(v0, v1);
+            } else {
+                p.out[at] = __float2bfloat16_rn(v0);
+                p.out[at + 1] = __float2bfloat16_rn(v1);
+            }
         } else if (p.cluster_merge) {
             const uint32_t at = incoming + (uint32_t)((cluster_rank * rows + r) * (HD + 2)) * 4u;
-            asm volatile("st.shared::cluster.f32 [%0], %1;\n" ::"r"(at + (uint32_t)d * 4u), "f"(a) : "memory");
-            if (d == 0) {
-                asm volatile("st.shared::cluster.f32 [%0], %1;\n" ::"r"(at + (uint32_t)HD * 4u), "f"(m) : "memory");
-                asm volatile("st.shared::cluster.f32 [%0], %1;\n" ::"r"(at + (uint32_t)(HD + 1) * 4u), "f"(l) : "memory");
-            }
+            asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};\n" ::"r"(at + (uint32_t)d * 4u), "f"(a), "f"(b) : "memory");
+            if (d == 0) asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};\n" ::"r"(at + (uint32_t)HD * 4u), "f"(m), "f"(l) : "memory");
         } else {
             const size_t slot = ((size_t)t * p.num_heads + h) * p.splits + split;
-            p.partial_acc[slot * HD + d] = a;
-            if (d == 0) {
-                p.partial_ml[slot * 2] = m;
-                p.partial_ml[slot * 2 + 1] = l;
-            }
+            *reinterpret_cast<float2*>(p.partial_acc + slot * HD + d) = make_float2(a, b);
+            if (d == 0) *reinterpret_cast<float2*>(p.partial_ml + slot * 2) = make_float2(m, l);
         }
     }
     trace_scope.mark(4);
@@ -625,6 +631,12 @@ int launch(cudaStream_t stream, const Params& p, int tokens) {
     // 16 clusters are 112 CTAs and the step takes 1.59 ms with them, 1.45 with 256 four-warp CTAs.
     constexpr int WIDE_KEYS = HD <= 64 ? 32 : 16;                                // keys a warp of the eight-warp form takes of a tile
     const long long most_tiles = ((long long)p.table_stride * p.page_size + TILE_KEYS - 1) / TILE_KEYS;
+    constexpr long long wide_tiles = 8;
+    if constexpr (HD <= 128) if ((long long)grid.x * grid.y <= sm_count && most_tiles <= wide_tiles) {
+        Params whole = p;
+        whole.splits = 1;
+        return launch_with<HD, true, MASKED, 2, WIDE_KEYS>(stream, whole, dim3(grid.x, grid.y, 1));
+    }
     if constexpr (HD <= 128) if (ctas <= 2ll * sm_count && p.splits >= 4 && p.splits % 2 == 0) {
         for (int fewer = 0; fewer <= 2; ++fewer) {
             Params half = p;

@@ -717,7 +717,7 @@ private:
                 throw DeviceError("a step has more (token, KV head) pairs than the attention's ticket counters");
             counters = ctx.scratch->attention_counters.as<int>();
         }
-        launch_check(eg_attention_paged(ctx.stream, qkv.p, (int)qkv.ld, cache.k, cache.v, tables.block_table, tables.table_width, ctx.token_seq,
+        launch_check(eg_attention_paged(ctx.stream, qkv.p, (int)qkv.ld, cache.k, cache.v, tables.block_table, tables.table_width, ctx.all_decode ? nullptr : ctx.token_seq,
                                         ctx.positions, seq_context, attn.p, (int)attn.ld, acc, ml, tokens, heads_, kv_heads_, head_dim_, cache.page_size,
                                         cache.page_stride, cache.head_stride, cache.num_pages, window, scale_, splits, ctx.status, nullptr, 0, counters,
                                         plans::use_pdl(), nullptr, token_list), "attention_paged");

@@ -167,7 +167,7 @@ private:
                 throw DeviceError("a step has more (token, KV head) pairs than the attention's ticket counters");
             counters = ctx.scratch->attention_counters.as<int>();
         }
-        launch_check(eg_attention_paged_sink(ctx.stream, q.p, (int)q.ld, cache.k, cache.v, tables.block_table, tables.table_width, ctx.token_seq, ctx.positions,
+        launch_check(eg_attention_paged_sink(ctx.stream, q.p, (int)q.ld, cache.k, cache.v, tables.block_table, tables.table_width, ctx.all_decode ? nullptr : ctx.token_seq, ctx.positions,
                                              seq_context, attn.p, (int)attn.ld, acc, ml, tokens, heads_, kv_heads_, dk_, cache.page_size, cache.page_stride,
                                              cache.head_stride, cache.num_pages, window, scale_, splits, ctx.status, counters, plans::use_pdl(), token_list, sink_),
                      "attention_paged_sink");

@@ -190,7 +190,7 @@ public:
                         throw DeviceError("a step has more (token, KV head) pairs than the attention's ticket counters");
                     counters = ctx.scratch->attention_counters.as<int>();
                 }
-                launch_check(eg_attention_paged_masked(ctx.stream, q.p, (int)q.ld, cache.k, cache.v, tables.block_table, tables.table_width, ctx.token_seq,
+                launch_check(eg_attention_paged_masked(ctx.stream, q.p, (int)q.ld, cache.k, cache.v, tables.block_table, tables.table_width, ctx.all_decode ? nullptr : ctx.token_seq,
                                                        ctx.positions, ctx.query_tiles ? nullptr : ctx.seq_context, out, (int)out_dtype, (int)ldo, acc, ml, singles,
                                                        rows, key_heads, maps_, dk_, cache.page_size, cache.page_stride, cache.head_stride, cache.num_pages,
                                                        (int)window_, (int)chunk_, (int)keep_first_, scale_, softcap_, sinks, slopes, factor, splits, ctx.status, counters,
