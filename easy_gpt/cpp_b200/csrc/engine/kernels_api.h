@@ -23,6 +23,10 @@ int eg_embedding_gather(cudaStream_t stream, int dtype, const int* ids, const vo
 int eg_add_into_f32(cudaStream_t stream, float* residual, const void* delta, int delta_dtype, long long n);
 // engine_ops.cu
 int eg_convert_rows(cudaStream_t stream, const void* src, int src_dtype, void* dst, int dst_dtype, long long n);
+// gemm_batch.cu
+int eg_gemm_batch_takes(int epilogue, int N, int K, int head_dim);
+// gemm_batch.cu
+int eg_gemm_batch(cudaStream_t stream, int epilogue, int use_pdl, const void* W, long long ldw, const float* bias, int M, int N, int K, const void* x, long long ldx, float eps, const float* ss_in, int ss_parts, void* out, long long ldo, int num_heads, int num_kv_heads, int head_dim, const float* rotations, const int* slot_map, void* k_cache, void* v_cache, int page_size, long long page_stride, long long head_stride, long long pool_slots, float* resid, const float* gain_out, void* xn_out, float* ss_out, const void* prefetch, long long prefetch_bytes, int* status);
 // gemm_f32.cu
 int eg_gemm_f32_nt(cudaStream_t stream, const float* A, int lda, const float* W, int ldw, const float* bias, float* C, int ldc, int M, int N, int K);
 // gemm_skinny.cu

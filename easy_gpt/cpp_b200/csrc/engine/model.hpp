@@ -25,6 +25,8 @@ struct SubLayer {
     bool plain_pre_norm = false;        // x = x + part(norm(x)) with nothing behind the part: the shape whose add and norm the parts may fuse
     // whether the sub-layer in front may prepare this one's norm: the part must take a norm that is not computed yet
     bool takes_prepared_norm() const { return plain_pre_norm && (mixer ? mixer->accepts_pending_norm() : feed_forward->accepts_pending_norm()); }
+    // the same in steps of 17 to 64 tokens
+    bool takes_prepared_batch(bool writes) const { return takes_prepared_norm() && (mixer ? mixer->takes_prepared_batch(writes) : feed_forward->takes_prepared_batch()); }
     Part* part() const { return mixer ? static_cast<Part*>(mixer.get()) : static_cast<Part*>(feed_forward.get()); }
     std::vector<Part*> parts() const {
         std::vector<Part*> out;
@@ -80,6 +82,7 @@ public:
     }
     // the norm that a fused add + norm in front of this layer would have to be (nullptr: nothing in front may prepare it)
     const Norm* first_norm() const { return !parallel && sublayers.front().takes_prepared_norm() ? sublayers.front().norm.get() : nullptr; }
+    bool first_takes_prepared_batch(bool writes) const { return !parallel && sublayers.front().takes_prepared_batch(writes); }
 
     // The residual stream between layers: the buffer that holds it, a second buffer of its size, and what is still to be
     // added to it (a part's output, or two of them behind a parallel layer; the norm that comes next adds them).
@@ -223,7 +226,7 @@ public:
     // next_reads_stream: the layer that runs next starts with a sub-layer that reads the stream itself; a last sub-layer that
     // joins the stream through its norm may then leave the stream's rows in `work` for it (Stream::rows_ahead).
     Stream forward(StepContext& ctx, StepArenas& arenas, int* turn, Stream s, const CacheView& cache, void* work, void* work2, const Norm* next_norm,
-                   bool next_reads_stream = false) const {
+                   bool next_reads_stream = false, bool next_takes_batch = false) const {
         const int T = ctx.num_tokens;
         const bool rows_ahead = s.rows_ahead;
         s.rows_ahead = false;
@@ -247,7 +250,9 @@ public:
                 FollowingNorm follow;
                 const FollowingNorm* offer = nullptr;
                 const bool fuses = sub.mixer ? sub.mixer->fuses_following_norm() : sub.feed_forward->fuses_following_norm();
-                if (fuses && following && following->rms_parameters(&follow.gain, &follow.eps) && ctx.dtype == DType::BF16 && T > 0 && T <= fused_rows) {
+                const bool batch = T > fused_rows && plans::batch_tokens(ctx.dtype, T) &&
+                                   (i + 1 < sublayers.size() ? sublayers[i + 1].takes_prepared_batch(cache.writes) : next_takes_batch);
+                if (fuses && following && following->rms_parameters(&follow.gain, &follow.eps) && ctx.dtype == DType::BF16 && T > 0 && (T <= fused_rows || batch)) {
                     follow.norm = following;
                     follow.pending = &pending;
                     offer = &follow;
@@ -569,7 +574,9 @@ public:
             // the norm that the next entry starts with, unless something is added to the stream before it
             const Norm* next_norm = (i + 1 < order.size()) ? (order[i + 1].stream_add >= 0 ? nullptr : blocks[order[i + 1].layer]->first_norm()) : final_norm.get();
             const bool next_reads_stream = i + 1 < order.size() && order[i + 1].stream_add < 0 && blocks[order[i + 1].layer]->reads_stream_first();
-            s = blocks[order[i].layer]->forward(ctx, arenas, &turn, s, view(order[i].cache, order[i].writes_cache), work, work2, next_norm, next_reads_stream);
+            const bool next_takes_batch = i + 1 < order.size() ? blocks[order[i + 1].layer]->first_takes_prepared_batch(order[i + 1].writes_cache) : true;   // (the head finishes its norm from the residual)
+            s = blocks[order[i].layer]->forward(ctx, arenas, &turn, s, view(order[i].cache, order[i].writes_cache), work, work2, next_norm, next_reads_stream,
+                                                next_takes_batch);
         }
         ctx.arena = &arenas.step;                // the head's rows and logits live for the step
         if (num_rows <= 0) return nullptr;

@@ -204,18 +204,34 @@ public:
         return out;
     }
 
+    // The same for steps of 17 to 64 tokens (gemm_batch.cu), of prepared rows (norm) or, into the residual, of plain ones
+    bool batch_takes(int epilogue, int head_dim) const { return dtype == DType::BF16 && eg_gemm_batch_takes(epilogue, out_features, in_features, head_dim) > 0; }
+    void batch(const StepContext& ctx, int epilogue, int M, const Rows* x, const NormInFront* norm, void* out, long long ldo, const SkinnyRope* rope,
+               const float* rotations, float* follow_residual, const float* follow_gain, void* xn_out, float* ss_out) const {
+        const SkinnyRope none{}, &r = rope ? *rope : none;
+        launch_check(eg_gemm_batch(ctx.stream, epilogue, plans::use_pdl(), weight, in_features, bias_f32(), M, out_features, in_features,
+                                   norm ? norm->prepared_rows : x->p, norm ? in_features : x->ld, norm ? norm->eps : 0.f, norm ? norm->prepared_sums : nullptr,
+                                   norm ? norm->prepared_parts : 0, out, ldo, r.num_heads, r.num_kv_heads, r.head_dim, rotations, r.slot_map, r.k_cache, r.v_cache,
+                                   r.page_size, r.page_stride, r.head_stride, r.pool_slots, follow_residual, follow_gain, xn_out, ss_out,
+                                   epilogue == plans::EPI_RESID_NORM ? ctx.soon : nullptr, (long long)ctx.soon_bytes, ctx.status), "gemm_batch");
+    }
+
     // whether with_following_norm can run for this input (the decode kernel takes it)
     bool takes_following_norm(const Rows& x) const {
+        if (plans::batch_tokens(dtype, x.rows)) return batch_takes(plans::EPI_RESID_NORM, 0) && aligned(x);
         return dtype == DType::BF16 && plans::gemm_skinny_takes(dtype, x.rows, in_features) && x.rows <= plans::FUSED_NORM_MAX_TOKENS && aligned(x);
     }
     // The product, the add to the residual and the preparation of the norm that follows, in one kernel:
     // follow.residual() += x W^T + b (in place); returns a PreNormed for follow.norm.
     PreNormed with_following_norm(const StepContext& ctx, const Rows& x, const FollowingNorm& follow) const {
         const plans::SkinnyPlan plan = plans::skinny_plan(out_features, in_features);
-        const int parts = (out_features + plan.row_blocks * 16 - 1) / (plan.row_blocks * 16);
+        const bool many = x.rows > plans::SKINNY_MAX_TOKENS;
+        const int parts = many ? eg_gemm_batch_takes(plans::EPI_RESID_NORM, out_features, in_features, 0)
+                               : (out_features + plan.row_blocks * 16 - 1) / (plan.row_blocks * 16);
         void* xn = ctx.take_rows(x.rows, out_features, DType::BF16);
         float* ss = ctx.take<float>((size_t)parts * plans::skinny_padded_tokens(x.rows));
-        skinny(ctx, plans::EPI_RESID_NORM, x.rows, &x, nullptr, nullptr, 0, nullptr, follow.residual(), follow.gain, xn, ss, &plan);
+        if (many) batch(ctx, plans::EPI_RESID_NORM, x.rows, &x, nullptr, nullptr, 0, nullptr, nullptr, follow.residual(), follow.gain, xn, ss);
+        else skinny(ctx, plans::EPI_RESID_NORM, x.rows, &x, nullptr, nullptr, 0, nullptr, follow.residual(), follow.gain, xn, ss, &plan);
         return PreNormed{follow.norm, xn, ss, parts};
     }
 
@@ -533,6 +549,11 @@ public:
     CacheNeed cache_need() const override { return CacheNeed::paged(kv_heads_, head_dim_, window_); }
     bool accepts_pending_norm() const override { return true; }
     bool fuses_following_norm() const override { return true; }
+    bool takes_prepared_batch(bool writes) const override {
+        HalfRotation rot;
+        return writes && position && position->half_rotation(&rot) && rot.magnitude == 1.0f && rot.rotary_dim == head_dim_ &&
+               qkv_.batch_takes(plans::EPI_QKV_ROPE, head_dim_);
+    }
 
     // norm + QKV (+ bias, rotation, cache write); attention over the cache; output projection into the residual
     bool emit_fused(FusedBuilder& b, const float* gain, float eps, const CacheView& cache) const override {
@@ -633,7 +654,8 @@ public:
             const NormInFront norm = in.pending->fused();
             const SkinnyRope rope{heads_, kv_heads_, head_dim_, ctx.positions, tables.slot_map, cache.k, cache.v, rot.inv_freq, cache.page_size,
                                   cache.page_stride, cache.head_stride, pool_slots};
-            qkv_.skinny(ctx, plans::EPI_QKV_ROPE, T, nullptr, &norm, qkv.p, q_width, &rope, nullptr, nullptr, nullptr, nullptr);
+            if (T > plans::SKINNY_MAX_TOKENS) qkv_.batch(ctx, plans::EPI_QKV_ROPE, T, nullptr, &norm, qkv.p, q_width, &rope, rotation_table(ctx, rot), nullptr, nullptr, nullptr, nullptr);
+            else qkv_.skinny(ctx, plans::EPI_QKV_ROPE, T, nullptr, &norm, qkv.p, q_width, &rope, nullptr, nullptr, nullptr, nullptr);
         } else {
             const Rows x = in.pending ? in.pending->materialize() : in.rows;
             qkv = qkv_(ctx, x);
@@ -776,6 +798,7 @@ public:
     bool capturable() const override { return true; }
     bool accepts_pending_norm() const override { return !clamped_; }
     bool fuses_following_norm() const override { return !clamped_; }
+    bool takes_prepared_batch() const override { return !clamped_ && gate_up_.batch_takes(plans::EPI_SWIGLU, 0); }
 
     // norm + gate/up + SwiGLU; down projection into the residual
     bool emit_fused(FusedBuilder& b, const float* gain, float eps) const override {
@@ -838,7 +861,8 @@ public:
         if (in.pending && in.pending->fusable) {
             // decode: add + norm + gate/up product + SwiGLU in one kernel
             const NormInFront norm = in.pending->fused();
-            gate_up_.skinny(ctx, plans::EPI_SWIGLU, T, nullptr, &norm, act.p, inter_, nullptr, nullptr, nullptr, nullptr, nullptr);
+            if (T > plans::SKINNY_MAX_TOKENS) gate_up_.batch(ctx, plans::EPI_SWIGLU, T, nullptr, &norm, act.p, inter_, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr);
+            else gate_up_.skinny(ctx, plans::EPI_SWIGLU, T, nullptr, &norm, act.p, inter_, nullptr, nullptr, nullptr, nullptr, nullptr);
         } else {
             const Rows x = in.pending ? in.pending->materialize() : in.rows;
             if (plans::gemm_skinny_takes(dtype, T, hidden_) && Linear::aligned(x)) {

@@ -312,8 +312,8 @@ public:
         residual_after = residual;
         spare_after = spare;
         has_rms_ = norm->rms_parameters(&gain_, &eps_);
-        fusable = has_rms_ && rows == nullptr && ctx.dtype == DType::BF16 && tokens > 0 && tokens <= max_fused_rows &&
-                  (!delta.has_delta() || delta.dtype == DType::BF16);
+        fusable = has_rms_ && rows == nullptr && ctx.dtype == DType::BF16 && tokens > 0 &&
+                  (tokens <= max_fused_rows ? !delta.has_delta() || delta.dtype == DType::BF16 : delta.has_pre());
     }
     // the norm as a kernel of its own; returns the normalised rows (ctx.dtype)
     Rows materialize() {
@@ -460,6 +460,8 @@ public:
     Mixer(const Params& params, const std::string& prefix, std::shared_ptr<PositionEncoding> position) : Part(params, prefix), position(std::move(position)) {}
     virtual bool accepts_pending_norm() const { return false; }
     virtual bool fuses_following_norm() const { return false; }
+    // whether it takes prepared rows in steps of 17 to 64 tokens too; writes: it writes its cache
+    virtual bool takes_prepared_batch(bool /*writes*/) const { return false; }
     virtual CacheNeed cache_need() const { return CacheNeed(); }
     // x [T, hidden] normalised input -> delta [T, hidden], both in ctx.dtype
     virtual Delta forward(const StepContext& ctx, PartInput x, const CacheView& cache, const FollowingNorm* follow) = 0;
@@ -475,6 +477,7 @@ public:
     virtual const void* first_weights(size_t* /*bytes*/) const { return nullptr; }
     virtual bool accepts_pending_norm() const { return false; }
     virtual bool fuses_following_norm() const { return false; }
+    virtual bool takes_prepared_batch() const { return false; }      // as Mixer's
     virtual Delta forward(const StepContext& ctx, PartInput x, const FollowingNorm* follow) = 0;
     // For a sub-layer that reads the stream itself (no norm in front) and joins it through an RMS norm on its output: the
     // whole of  x += a + b (what is still to be added, each with its gain);  x += gain * y / rms(y), y = this(x)  in the part's

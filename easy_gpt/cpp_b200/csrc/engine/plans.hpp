@@ -145,6 +145,9 @@ inline SkinnyPlan skinny_plan(int n_rows, int in_features, int head_dim = 0) {
 inline bool gemm_skinny_takes(DType dtype, int tokens, int in_features) {
     return dtype == DType::BF16 && tokens > 0 && tokens <= SKINNY_MAX_TOKENS && in_features % 16 == 0;
 }
+// Steps of 17 to 64 tokens: rows that a product has prepared go from product to product (gemm_batch.cu) where the parts can say so.
+constexpr int BATCH_MAX_TOKENS = 64;
+inline bool batch_tokens(DType dtype, int tokens) { return dtype == DType::BF16 && tokens > SKINNY_MAX_TOKENS && tokens <= BATCH_MAX_TOKENS; }
 inline int skinny_padded_tokens(int tokens) { return tokens <= 8 ? 8 : tokens <= 16 ? 16 : tokens <= 32 ? 32 : 64; }
 
 // How much of the feed-forward's first matrix the output projection in front of it asks the L2 for: what arrives while the
