@@ -564,15 +564,29 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
         if (lane == 0) {                                         // ---- TMA producer, in both CTAs
             int g = 0;
             bool ok = true;
+            // the weights of the first tile's first stages are asked for before the kernel in front is known to be done
+            const int early = min(PSTAGES, k_blocks);
+            {
+                const int n0 = (pair / m_tiles) * PBN + rank * (PBN / 2);
+                for (int kb = 0; kb < early; ++kb) {
+                    if (rank == 0) mbar_expect_tx(&full_bar[kb], 2 * P_STAGE_BYTES);
+                    unsigned char* w = ring + kb * P_STAGE_BYTES + 2 * C::A_SUB_BYTES;
+                    tma_load_2d_pair(w, &map_w, &full_bar[kb], kb * PBK, n0);
+                    tma_load_2d_pair(w + C::W_SUB_BYTES, &map_w, &full_bar[kb], kb * PBK + BK, n0);
+                }
+            }
+            asm volatile("griddepcontrol.wait;\n" ::: "memory");
+            asm volatile("griddepcontrol.launch_dependents;\n" ::);
             for (int t = pair; t < total_tiles && ok; t += pairs) {
                 const int n0 = (t / m_tiles) * PBN + rank * (PBN / 2), m0 = (t % m_tiles) * 2 * BM + rank * BM;
                 for (int kb = 0; kb < k_blocks; ++kb, ++g) {
                     const int s = g % PSTAGES;
                     if (g >= PSTAGES && !mbar_wait(&empty_bar[s], ((g / PSTAGES) - 1) & 1, &abort_flag, p.status)) { ok = false; break; }
-                    if (rank == 0) mbar_expect_tx(&full_bar[s], 2 * P_STAGE_BYTES);
+                    if (rank == 0 && g >= early) mbar_expect_tx(&full_bar[s], 2 * P_STAGE_BYTES);
                     unsigned char* a = ring + s * P_STAGE_BYTES;
                     tma_load_2d_pair(a, &map_a, &full_bar[s], kb * PBK, m0);
                     tma_load_2d_pair(a + C::A_SUB_BYTES, &map_a, &full_bar[s], kb * PBK + BK, m0);
+                    if (g < early) continue;
                     tma_load_2d_pair(a + 2 * C::A_SUB_BYTES, &map_w, &full_bar[s], kb * PBK, n0);
                     tma_load_2d_pair(a + 2 * C::A_SUB_BYTES + C::W_SUB_BYTES, &map_w, &full_bar[s], kb * PBK + BK, n0);
                 }
@@ -1135,7 +1149,7 @@ int launch_pair(cudaStream_t stream, const CUtensorMap& map_a, const CUtensorMap
     }
     const int tiles = ((p.M + 2 * BM - 1) / (2 * BM)) * (p.N / PBN);
     const int pairs = tiles < sm_count / 2 ? tiles : sm_count / 2;
-    pairk::gemm_tcgen05_pair_kernel<PBN><<<2 * pairs, pairk::PTHREADS, C::SMEM_BYTES, stream>>>(map_a, map_w, map_out, p);
+    eg_pdl_launch(pairk::gemm_tcgen05_pair_kernel<PBN>, dim3(2 * pairs), dim3(pairk::PTHREADS), (size_t)C::SMEM_BYTES, stream, map_a, map_w, map_out, p);
     return eg_launch_status();
 }
 }  // namespace
