@@ -79,7 +79,7 @@ __device__ __forceinline__ void consumers_sync() { asm volatile("bar.sync 1, %0;
 template <int NT, int EPI, int NORM, bool GIVE_UP>
 __global__ void __launch_bounds__(THREADS, 2)
 stream_kernel(const Params p, const Plan s, const __grid_constant__ CUtensorMap unit_map, const __grid_constant__ CUtensorMap block_map) {
-    constexpr int MT = NT * 8, AT_ONCE = NT == 1 ? 2 : 1;
+    constexpr int MT = NT * 8;
     extern __shared__ unsigned char smem_raw[];
     unsigned char* smem = smem_raw + ((1024u - (smem_addr(smem_raw) & 1023u)) & 1023u);      // swizzled tiles start on 1,024 bytes
     __shared__ __align__(8) uint64_t full[MAX_STAGES], empty[MAX_STAGES], factor_bar, parts_bar;
@@ -274,60 +274,42 @@ stream_kernel(const Params p, const Plan s, const __grid_constant__ CUtensorMap 
     };
     for (int unit = 0; unit < units; ++unit) {
         const int rows = rows_of(unit);
-        // Four sums side by side, one for each 16 terms of a tile, that meet behind the last stage: a product's latency then counts once a
-        // stage and not four times.  Two stages at a time: their loads are under way together, and their products follow.
-        float acc[4][NT][4];
+        float acc[NT][4];
 #pragma unroll
-        for (int j = 0; j < 4; ++j)
+        for (int i = 0; i < NT; ++i) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.f;
+        for (int st = 0; st < k_stages; ++st) {
+            ok = ok && wait_for(&full[slot], phase, &abort_flag, p.status);
+            const int k = st * kc + ks * 64;
+            if (rb * 16 < rows && k < k_len) {
+                // all loads of the tile first: the products then follow one another without a trip to shared memory between them
+                const uint32_t w_at = (uint32_t)slot * STAGE_BYTES, x_at = x_lane + (uint32_t)k * 2;
+                uint32_t a[4][4], b[4][NT][2];
 #pragma unroll
-            for (int i = 0; i < NT; ++i) acc[j][i][0] = acc[j][i][1] = acc[j][i][2] = acc[j][i][3] = 0.f;
-        for (int st = 0; st < k_stages; st += AT_ONCE) {
-            uint32_t a[AT_ONCE][4][4], b[AT_ONCE][4][NT][2];
-            bool mine[AT_ONCE];
-            int at_slot[AT_ONCE];
+                for (int j = 0; j < 4; ++j) {
+                    ldmatrix4(a[j], w_step[j] + w_at);
+                    if (NT == 1) {
+                        ldmatrix2(b[j][0][0], b[j][0][1], x_at + j * 32);
+                    } else {
 #pragma unroll
-            for (int h = 0; h < AT_ONCE; ++h) {
-                const int k = (st + h) * kc + ks * 64;
-                at_slot[h] = slot;
-                mine[h] = false;
-                if (st + h >= k_stages) continue;
-                ok = ok && wait_for(&full[slot], phase, &abort_flag, p.status);
-                mine[h] = rb * 16 < rows && k < k_len;
-                if (mine[h]) {
-                    const uint32_t w_at = (uint32_t)slot * STAGE_BYTES, x_at = x_lane + (uint32_t)k * 2;
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) {
-                        ldmatrix4(a[h][j], w_step[j] + w_at);
-                        if (NT == 1) {
-                            ldmatrix2(b[h][j][0][0], b[h][j][0][1], x_at + j * 32);
-                        } else {
-#pragma unroll
-                            for (int nt = 0; nt + 1 < NT; nt += 2) {
-                                uint32_t t[4];
-                                ldmatrix4(t, x_at + nt * 8 * x_stride + j * 32);
-                                b[h][j][nt][0] = t[0];
-                                b[h][j][nt][1] = t[1];
-                                b[h][j][nt + 1][0] = t[2];
-                                b[h][j][nt + 1][1] = t[3];
-                            }
+                        for (int nt = 0; nt + 1 < NT; nt += 2) {
+                            uint32_t t[4];
+                            ldmatrix4(t, x_at + nt * 8 * x_stride + j * 32);
+                            b[j][nt][0] = t[0];
+                            b[j][nt][1] = t[1];
+                            b[j][nt + 1][0] = t[2];
+                            b[j][nt + 1][1] = t[3];
                         }
                     }
                 }
-                if (++slot == s.stages) { slot = 0; phase ^= 1u; }
+#pragma unroll
+                for (int j = 0; j < 4; ++j)
+                    if (k + j * 16 < k_len)                       // (behind it x is another row's or nobody's memory)
+#pragma unroll
+                        for (int nt = 0; nt < NT; ++nt) mma_bf16_16816(acc[nt], a[j], b[j][nt][0], b[j][nt][1]);
             }
-#pragma unroll
-            for (int h = 0; h < AT_ONCE; ++h) {
-                const int k = (st + h) * kc + ks * 64;
-                if (mine[h])
-#pragma unroll
-                    for (int j = 0; j < 4; ++j)
-                        if (k + j * 16 < k_len)                   // (behind it x is another row's or nobody's memory)
-#pragma unroll
-                            for (int nt = 0; nt < NT; ++nt) mma_bf16_16816(acc[j][nt], a[h][j], b[h][j][nt][0], b[h][j][nt][1]);
-                if (st + h >= k_stages) continue;
-                __syncwarp();
-                if (lane == 0 && ok) mbar_arrive(&empty[at_slot[h]]);      // (who gave up has not seen the stage full: it is not asked for again)
-            }
+            __syncwarp();
+            if (lane == 0 && ok) mbar_arrive(&empty[slot]);       // (who gave up has not seen the stage full: it is not asked for again)
+            if (++slot == s.stages) { slot = 0; phase ^= 1u; }
         }
         if (unit == 0) {
             trace_scope.mark(3, true);
@@ -340,10 +322,10 @@ stream_kernel(const Params p, const Plan s, const __grid_constant__ CUtensorMap 
 #pragma unroll
         for (int nt = 0; nt < NT; ++nt) {
             float* base = red + ((size_t)warp * MT + nt * 8 + 2 * tig) * RED_LD + gid;
-            base[0] = (acc[0][nt][0] + acc[1][nt][0]) + (acc[2][nt][0] + acc[3][nt][0]);
-            base[RED_LD] = (acc[0][nt][1] + acc[1][nt][1]) + (acc[2][nt][1] + acc[3][nt][1]);
-            base[8] = (acc[0][nt][2] + acc[1][nt][2]) + (acc[2][nt][2] + acc[3][nt][2]);
-            base[RED_LD + 8] = (acc[0][nt][3] + acc[1][nt][3]) + (acc[2][nt][3] + acc[3][nt][3]);
+            base[0] = acc[nt][0];
+            base[RED_LD] = acc[nt][1];
+            base[8] = acc[nt][2];
+            base[RED_LD + 8] = acc[nt][3];
         }
         consumers_sync();
         trace_scope.mark(4);
