@@ -47,7 +47,6 @@ attention_generic_kernel(const T* __restrict__ q, int ldq, const T* __restrict__
                          const int* __restrict__ positions, T* __restrict__ out, int ldo, int num_heads, int num_kv_heads,
                          int head_dim, int page_size, long long page_stride, long long head_stride, int num_pages,
                          int window, float scale, int* status) {
-    pdl_enter();
     extern __shared__ __align__(16) float smem[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
     const int t = blockIdx.x, kvh = blockIdx.y, group = num_heads / num_kv_heads;
@@ -208,8 +207,8 @@ int launch_generic(cudaStream_t stream, const T* q, int ldq, const T* k, const T
     static const cudaError_t configured = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
     if (configured != cudaSuccess) return (int)configured;
     const dim3 grid(tokens, num_kv_heads, (num_heads / num_kv_heads + HG - 1) / HG);
-    eg_pdl_launch(kernel, grid, dim3(warps * 32), bytes, stream, q, ldq, k, v, table, table_stride, token_seq, positions, out, ldo, num_heads, num_kv_heads, head_dim,
-                  page_size, page_stride, head_stride, num_pages, window, scale, status);
+    kernel<<<grid, warps * 32, bytes, stream>>>(q, ldq, k, v, table, table_stride, token_seq, positions, out, ldo, num_heads, num_kv_heads, head_dim, page_size,
+                                                page_stride, head_stride, num_pages, window, scale, status);
     return eg_launch_status();
 }
 

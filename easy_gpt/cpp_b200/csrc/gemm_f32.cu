@@ -96,8 +96,9 @@ f32_rows_kernel(const float* __restrict__ A, int lda, const float* __restrict__ 
     float* stages = smem + warp * 2 * RowsMemory<BM>::STAGE;
     const int chunks = (last - first + CHUNK - 1) / CHUNK;
 
-    auto weights = [&](int c) {
+    auto stage = [&](int c) {
         float* ws = stages + (c & 1) * RowsMemory<BM>::STAGE;
+        float* xs = ws + ROWS * W_STRIDE;
         const int k0 = first + c * CHUNK;
         if (VEC) {
 #pragma unroll
@@ -112,10 +113,6 @@ f32_rows_kernel(const float* __restrict__ A, int lda, const float* __restrict__ 
                 copy4(ws + row * W_STRIDE + lane, in ? W + (size_t)(n0 + row) * ldw + k0 + lane : W, in ? 4 : 0);
             }
         }
-    };
-    auto inputs = [&](int c) {                         // and what has been asked for until here is one group
-        float* xs = stages + (c & 1) * RowsMemory<BM>::STAGE + ROWS * W_STRIDE;
-        const int k0 = first + c * CHUNK;
 #pragma unroll
         for (int m = 0; m < BM; ++m) {
             const bool in = m < M && k0 + lane < last;
@@ -127,15 +124,10 @@ f32_rows_kernel(const float* __restrict__ A, int lda, const float* __restrict__ 
     f32x2 acc[2][BM / 2];
 #pragma unroll
     for (int m = 0; m < BM / 2; ++m) acc[0][m] = acc[1][m] = 0ull;
-    // both stages' weights are on their way before the kernel in front is known to be done
-    if (chunks > 0) weights(0);
-    if (chunks > 1) weights(1);
-    pdl_enter();
-    if (chunks > 0) inputs(0);
+    if (chunks > 0) stage(0);
     for (int c = 0; c < chunks; ++c) {
         if (c + 1 < chunks) {
-            if (c > 0) weights(c + 1);
-            inputs(c + 1);
+            stage(c + 1);
             asm volatile("cp.async.wait_group 1;\n" ::: "memory");
         } else {
             asm volatile("cp.async.wait_group 0;\n" ::: "memory");
@@ -227,7 +219,6 @@ f32_tile_kernel(const float* __restrict__ A, int lda, const float* __restrict__ 
     const int ctas = split ? groups : 1;
     const int my_group = blockIdx.x % ctas, n0 = blockIdx.x / ctas * BN, m0 = blockIdx.y * BM;
 
-    pdl_enter();
     float4 a_next[A_LOADS], w_next[W_LOADS];
     auto fetch = [&](int k0) {
         auto piece = [&](const float* base, int ld, int row, int rows, int k) {
@@ -380,15 +371,12 @@ int launch_clusters(Kernel kernel, dim3 grid, int threads, int smem, int cluster
     cfg.blockDim = dim3(threads);
     cfg.dynamicSmemBytes = (size_t)smem;
     cfg.stream = stream;
-    static const bool early = !(getenv("EASY_GPT_PDL") && atoi(getenv("EASY_GPT_PDL")) == 0);
-    cudaLaunchAttribute attr[2];
+    cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = (unsigned)cluster;
     attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
-    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = early ? 2 : 1;
+    cfg.numAttrs = 1;
     e = cudaLaunchKernelEx(&cfg, kernel, args...);
     return e != cudaSuccess ? (int)e : eg_launch_status();
 }
