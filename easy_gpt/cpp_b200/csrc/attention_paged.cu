@@ -631,8 +631,12 @@ int launch(cudaStream_t stream, const Params& p, int tokens) {
     // 16 clusters are 112 CTAs and the step takes 1.59 ms with them, 1.45 with 256 four-warp CTAs.
     constexpr int WIDE_KEYS = HD <= 64 ? 32 : 16;                                // keys a warp of the eight-warp form takes of a tile
     const long long most_tiles = ((long long)p.table_stride * p.page_size + TILE_KEYS - 1) / TILE_KEYS;
-    constexpr long long wide_tiles = 8;
-    if constexpr (HD <= 128) if ((long long)grid.x * grid.y <= sm_count && most_tiles <= wide_tiles) {
+    // Short contexts: the eight-warp form takes four tiles of heads of 64 (two of 128) at a time, so a CTA walks a context of 512 in two (four)
+    // rounds by itself, and nothing is merged across CTAs.  Heads of 128 only where the launch has 16 pairs and more: fewer are better
+    // off in two CTAs each.  (us a decode step, two four-warp CTAs / one of eight warps: 0.5B sizes, 300 keys, batch 1 / 8 / 16, 592 / 636 /
+    // 739 and 593 / 630 / 727; up to 1,024 keys, 700 of them, batch 1, 593 and 624; 1.5B sizes, 300 keys, 1,088 / 1,194 / 1,347 and 1,100 /
+    // 1,193 / 1,314.)
+    if constexpr (HD <= 128) if (most_tiles <= 8 && (long long)grid.x * grid.y <= sm_count && (HD <= 64 || grid.x * grid.y >= 16)) {
         Params whole = p;
         whole.splits = 1;
         return launch_with<HD, true, MASKED, 2, WIDE_KEYS>(stream, whole, dim3(grid.x, grid.y, 1));
