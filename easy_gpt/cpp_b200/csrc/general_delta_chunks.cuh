@@ -127,38 +127,40 @@ __global__ void __launch_bounds__(128) general_delta_chunks_kernel(const DeltaPa
     if (tid < CHUNK_DIM) {
         // ---- a channel's X and R - Q X
         const int c = tid;
-        float x[CHUNK], run = 1.f;
+        // (running products in 64 bits: rounded once, they add nothing to what a step by step product of the decays would lose)
+        float x[CHUNK];
+        double run = 1.0;
 #pragma unroll
         for (int t = 0; t < CHUNK; ++t) {
-            x[t] = su[t][c] * run;
+            x[t] = (float)(su[t][c] * run);
             run *= sw[t][c];
 #pragma unroll
             for (int j = 0; j < t; ++j) x[t] = fmaf(-coef[0][t][j], x[j], x[t]);
         }
 #pragma unroll
         for (int t = 0; t < CHUNK; t += 4) *reinterpret_cast<float4*>(rec + c * CHUNK + t) = make_float4(x[t], x[t + 1], x[t + 2], x[t + 3]);
-        run = 1.f;
+        run = 1.0;
 #pragma unroll
         for (int t = 0; t < CHUNK; t += 4) {
             float o[4];
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
                 run *= sw[t + e][c];
-                o[e] = sr[t + e][c] * run;
+                o[e] = (float)(sr[t + e][c] * run);
 #pragma unroll
                 for (int j = 0; j <= t + e; ++j) o[e] = fmaf(-coef[3][t + e][j], x[j], o[e]);
             }
             *reinterpret_cast<float4*>(rec + CHUNK * CHUNK_DIM + c * CHUNK + t) = make_float4(o[0], o[1], o[2], o[3]);
         }
-        rec[4 * CHUNK * CHUNK_DIM + c] = run;
+        rec[4 * CHUNK * CHUNK_DIM + c] = (float)run;
     } else {
         // ---- a channel's D and K, and a column's V, H0 and P V - Q H0
         const int c = tid - CHUNK_DIM;
-        float run = 1.f;
+        double run = 1.0;
 #pragma unroll
         for (int t = CHUNK - 1; t >= 0; --t) {
-            rec[2 * CHUNK * CHUNK_DIM + t * CHUNK_DIM + c] = sa[t][c] * run;
-            rec[3 * CHUNK * CHUNK_DIM + t * CHUNK_DIM + c] = sk[t][c] * run;
+            rec[2 * CHUNK * CHUNK_DIM + t * CHUNK_DIM + c] = (float)(sa[t][c] * run);
+            rec[3 * CHUNK * CHUNK_DIM + t * CHUNK_DIM + c] = (float)(sk[t][c] * run);
             run *= sw[t][c];
         }
         float* slice = rec + CHUNK_SHARED + c / CHUNK_COLS * CHUNK_SLICE + c % CHUNK_COLS;
