@@ -141,6 +141,7 @@ __global__ void __launch_bounds__(1024) gated_delta_kernel(const float* __restri
                                                            const int* __restrict__ seq_slots, TO* __restrict__ y, long long ldy,
                                                            float* __restrict__ o_raw, int cols, int heads, int kv_heads, int dk, int dv, float eps,
                                                            int wide, const float* __restrict__ decay, long long ldg, int gate_sigmoid, float out_scale) {
+    pdl_enter();
     extern __shared__ __align__(16) float smem[];
     constexpr int RS = R + PAD, DKS = RS * P;       // a part's stride, a staged row's length (rows beyond dk hold zeros)
     constexpr int VECS = CH ? 3 : 2;                // staged vectors of dk values a token: key, query and, with CH, decay
@@ -155,26 +156,13 @@ __global__ void __launch_bounds__(1024) gated_delta_kernel(const float* __restri
     const bool active = jl < width;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
     float* S = state + (size_t)seq_slots[seq] * slot_floats + state_offset + ((size_t)head * dv + (active ? j : 0)) * dk;
-    // The state is what an earlier step left (or an earlier layer's kernel, which the one in front has waited for): it comes while the
-    // kernel in front still runs, in pieces of four rows where they start on 16-byte boundaries.
-    const bool quads = R % 4 == 0 && dk % 4 == 0 && slot_floats % 4 == 0 && state_offset % 4 == 0 && (uintptr_t)state % 16 == 0;
     float s[R];
-    if (quads) {
 #pragma unroll
-        for (int r = 0; r + 4 <= R; r += 4) {
-            const int row = part * R + r;
-            const float4 f = active && row < dk ? *reinterpret_cast<const float4*>(S + row) : make_float4(0.f, 0.f, 0.f, 0.f);
-            s[r] = f.x; s[r + 1] = f.y; s[r + 2] = f.z; s[r + 3] = f.w;
-        }
-    } else {
-#pragma unroll
-        for (int r = 0; r < R; ++r) {
-            const int row = part * R + r;
-            s[r] = (active && row < dk) ? S[row] : 0.f;
-        }
+    for (int r = 0; r < R; ++r) {
+        const int row = part * R + r;
+        s[r] = (active && row < dk) ? S[row] : 0.f;
     }
     for (int i = threadIdx.x; i < 2 * stage_floats; i += blockDim.x) smem[i] = 0.f;      // rows beyond dk stay zero
-    pdl_enter();
     __syncthreads();
     // tile `ti` into buffer `b`: 16-byte pieces where every row starts on a 16-byte boundary (wide), else value by value
     auto fetch = [&](int ti, int b) {
@@ -293,11 +281,7 @@ __global__ void __launch_bounds__(1024) gated_delta_kernel(const float* __restri
                 out[d] = from_f32<TO>(s_o[t * cols + d] * inv * norm_w[d] * (gate_sigmoid ? 1.0f / (1.0f + expf(-z[d])) : silu_f(z[d])) * out_scale);
         }
     }
-    if (active && quads) {
-#pragma unroll
-        for (int r = 0; r + 4 <= R; r += 4)
-            if (part * R + r < dk) *reinterpret_cast<float4*>(S + part * R + r) = make_float4(s[r], s[r + 1], s[r + 2], s[r + 3]);
-    } else if (active) {
+    if (active) {
 #pragma unroll
         for (int r = 0; r < R; ++r) {
             const int row = part * R + r;

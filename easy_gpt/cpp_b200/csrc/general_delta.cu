@@ -278,7 +278,7 @@ __global__ void __launch_bounds__(256) general_delta_output_kernel(const DeltaPa
 // INLINE: the block makes its entry's records itself (entries of up to p.tile tokens)
 template <typename TO, int R, int P, int COLS, bool INLINE>
 __global__ void __launch_bounds__(INLINE ? 512 : 256, 1) general_delta_kernel(const DeltaParams p) {
-    if (!INLINE) pdl_enter();                       // the records come from the kernel in front
+    pdl_enter();
     extern __shared__ __align__(128) float smem[];
     __shared__ __align__(8) uint64_t full[STAGES];
     __shared__ int abort_flag;
@@ -323,7 +323,6 @@ __global__ void __launch_bounds__(INLINE ? 512 : 256, 1) general_delta_kernel(co
             s[c][2 * i] = pair_of(v[0], v[1]);
             s[c][2 * i + 1] = pair_of(v[2], v[3]);
         }
-    if (INLINE) pdl_enter();                        // (the state is what an earlier step or layer left: it comes while the kernel in front still runs)
     if (INLINE && count > TILE) {                   // the host hands no such step here
         if (threadIdx.x == 0) atomicOr(p.status, EG_STATUS_BAD_SLOT);
         return;
