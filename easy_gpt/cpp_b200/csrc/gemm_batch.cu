@@ -10,7 +10,7 @@
 //   sums      CTAs that share a K range are a cluster; each owns BN / CS of the columns and gets the others' parts of them by
 //             st.async, counted on its mbarrier, and adds them up in their order.
 //   prologue  plain rows, or rows prepared by the product in front with partial sums of squares [token][part].
-//   epilogues a thread has half of a token's columns: into the residual with the next norm's preparation, SwiGLU of interleaved rows, or bias,
+//   epilogues a thread has a token: into the residual with the next norm's preparation, SwiGLU of interleaved rows, or bias,
 //             rotation and cache write (a tile is a head).
 //
 // Bound by the chain of latencies behind the wait (x, the products, the exchange) and by the weights' stream; 14 to 152 column
@@ -24,7 +24,7 @@ namespace {
 using namespace skinny;
 using batch_plan::BK;
 
-constexpr int THREADS = 192;                  // four warps of tokens, one that copies, one that multiplies
+constexpr int THREADS = 192;                  // two warps of tokens, one that copies, one that multiplies, two that help with the sums of squares
 constexpr unsigned PARTS_WAIT_LIMIT = WAIT_LIMIT << 7;
 constexpr int PREFETCH_PIECE = 16 * 1024;
 
@@ -93,7 +93,7 @@ batch_kernel(const Params p, const Plan s, const float2* __restrict__ rotations,
     float* parts = reinterpret_cast<float*>(ring + s.stages * Z::STAGE);                     // [CS][MT][PART_LD]
     __shared__ __align__(8) uint64_t full[batch_plan::MAX_STAGES], empty[batch_plan::MAX_STAGES], sums_bar, parts_bar;
     __shared__ uint32_t tmem_slot;
-    __shared__ float squares[2][64];
+    __shared__ float squares[64];
     __shared__ volatile int abort_flag, asked;                    // asked: stages that have been asked for, once the copying thread is done
     TraceScope trace_scope(p.trace);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -179,10 +179,9 @@ batch_kernel(const Params p, const Plan s, const float2* __restrict__ rotations,
             if (ok) commit(&sums_bar);
         }
     } else {
-        // ---- the tokens' epilogue: warps 0, 1 and 4, 5 (TMEM lanes 0 .. 63, twice: half of the columns each).  Loops stay rolled: in
-        // kernels this short the code that is walked for the first time is what the clock sees (40 ns for eight instructions).
-        const int m = threadIdx.x & 63, second = threadIdx.x >= 128;
-        const bool has_token = m < p.M;
+        // ---- the tokens' epilogue: warps 0 and 1 (TMEM lanes 0 .. 63), helped by 4 and 5
+        const int m = threadIdx.x < 64 ? threadIdx.x : threadIdx.x - 128;
+        const bool has_token = m < p.M, helper = threadIdx.x >= 64;
         float factor = 1.f;
         if (NORM == 2) {
             // the partial sums of squares of a token, every other four of them a thread, always in the same order
@@ -190,51 +189,52 @@ batch_kernel(const Params p, const Plan s, const float2* __restrict__ rotations,
             if (has_token) {
                 const float4* from = reinterpret_cast<const float4*>(p.ss_in + (size_t)m * p.ss_parts);
 #pragma unroll 8
-                for (int q = second; q < p.ss_parts / 4; q += 2) {
+                for (int q = helper; q < p.ss_parts / 4; q += 2) {
                     const float4 v = __ldcg(from + q);
                     ss.x += v.x; ss.y += v.y; ss.z += v.z; ss.w += v.w;
                 }
             }
-            squares[second][m] = (ss.x + ss.y) + (ss.z + ss.w);
+            const float sum = (ss.x + ss.y) + (ss.z + ss.w);
+            if (helper) squares[m] = sum;
             asm volatile("bar.sync 1, 128;\n" ::: "memory");
-            factor = 1.0f / sqrtf((squares[0][m] + squares[1][m]) / (float)p.K + p.eps);
+            if (!helper) factor = 1.0f / sqrtf((sum + squares[m]) / (float)p.K + p.eps);
         }
-        const int quad = warp & 3;
-        if (quad * 32 < MT) {
+        if (!helper && warp * 32 < MT) {
             constexpr int OWN = Z::OWN;
             // EPI_QKV_ROPE: a tile is a head; rank r of CS owns an even share of its pairs (j, j + half)
             constexpr int half = BN / 2, share = OWN / 2;
-            // EPI_RESID_NORM: eight columns a thread, the residual's asked for here, so that their trip runs beside the product
-            constexpr int PIECE = 8;
-            const bool resid_mine = EPI == EPI_RESID_NORM && has_token && (OWN > PIECE || !second);
-            const int resid_at = n0 + rank * OWN + (OWN > PIECE ? second * PIECE : 0);
-            float4 resid0, resid1;
-            if (resid_mine) {
-                const float4* from = reinterpret_cast<const float4*>(p.resid_inout + (size_t)m * p.N + resid_at);
-                resid0 = from[0];
-                resid1 = from[1];
+            // the residual's share is asked for here, so that its trip runs beside the product
+            float v[OWN], resid[EPI == EPI_RESID_NORM ? OWN : 1];
+            if (EPI == EPI_RESID_NORM && has_token) {
+                const float4* from = reinterpret_cast<const float4*>(p.resid_inout + (size_t)m * p.N + n0 + rank * OWN);
+#pragma unroll
+                for (int i = 0; i < OWN / 4; ++i) {
+                    const float4 f = from[i];
+                    resid[4 * i] = f.x; resid[4 * i + 1] = f.y; resid[4 * i + 2] = f.z; resid[4 * i + 3] = f.w;
+                }
             }
             const bool summed = __all_sync(0xffffffffu, wait_for(&sums_bar, 0, &abort_flag, p.status));
             trace_scope.mark(3);
             asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-            const uint32_t mine = tmem + ((uint32_t)(quad * 32) << 16);
-            ok = summed;
+            const uint32_t mine = tmem + ((uint32_t)(warp * 32) << 16);
             if (CS > 1) {
                 const uint32_t to = smem_addr(parts + ((size_t)rank * MT + m) * Z::PART_LD), bar = smem_addr(&parts_bar);
-#pragma unroll 1
-                for (int c0 = second * half; c0 < second * half + half; c0 += 16) {
+                uint32_t far[CS], far_bar[CS];
+#pragma unroll
+                for (int o = 0; o < CS; ++o) {
+                    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(far[o]) : "r"(to), "r"(o));
+                    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(far_bar[o]) : "r"(bar), "r"(o));
+                }
+#pragma unroll
+                for (int c0 = 0; c0 < BN; c0 += 16) {
                     float t[16];
                     tmem_16(mine + c0, t);
 #pragma unroll
-                    for (int i = 0; i < 16; i += 4) {
-                        const int c = c0 + i, jj = c & (half - 1);
-                        const int o = EPI == EPI_QKV_ROPE ? jj / share : c / OWN, place = EPI == EPI_QKV_ROPE ? second * share + jj % share : c % OWN;
-                        uint32_t far, far_bar;
-                        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(far) : "r"(to), "r"(o));
-                        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(far_bar) : "r"(bar), "r"(o));
+                    for (int c = c0; c < c0 + 16; c += 4) {
+                        const int jj = c % half, o = EPI == EPI_QKV_ROPE ? jj / share : c / OWN, place = EPI == EPI_QKV_ROPE ? c / half * share + jj % share : c % OWN;
                         asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1, %2, %3, %4}, [%5];\n"
-                                     ::"r"(far + (uint32_t)place * 4u), "r"(__float_as_uint(t[i])), "r"(__float_as_uint(t[i + 1])), "r"(__float_as_uint(t[i + 2])),
-                                       "r"(__float_as_uint(t[i + 3])), "r"(far_bar) : "memory");
+                                     ::"r"(far[o] + (uint32_t)place * 4u), "r"(__float_as_uint(t[c - c0])), "r"(__float_as_uint(t[c - c0 + 1])),
+                                       "r"(__float_as_uint(t[c - c0 + 2])), "r"(__float_as_uint(t[c - c0 + 3])), "r"(far_bar[o]) : "memory");
                     }
                 }
                 // (The others send their parts whatever became of their own waits, at most one limit a stage later: this CTA must
@@ -243,86 +243,76 @@ batch_kernel(const Params p, const Plan s, const float2* __restrict__ rotations,
                 for (unsigned i = 0; i < PARTS_WAIT_LIMIT && !landed; ++i) landed = try_wait_cluster(&parts_bar, 0);
                 if (!landed && p.status) atomicOr(p.status, EG_STATUS_WAIT_TIMEOUT);
                 ok = summed && __all_sync(0xffffffffu, landed);
+#pragma unroll
+                for (int i = 0; i < OWN; i += 4) {
+                    float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+                    for (int o = 0; o < CS; ++o) {
+                        const float4 f = *reinterpret_cast<const float4*>(parts + ((size_t)o * MT + m) * Z::PART_LD + i);
+                        sum.x += f.x; sum.y += f.y; sum.z += f.z; sum.w += f.w;
+                    }
+                    v[i] = sum.x; v[i + 1] = sum.y; v[i + 2] = sum.z; v[i + 3] = sum.w;
+                }
+            } else {
+                ok = summed;
+#pragma unroll
+                for (int c0 = 0; c0 < OWN; c0 += 16) {
+                    float t[16];
+                    tmem_16(mine + c0, t);
+#pragma unroll
+                    for (int i = 0; i < 16; ++i) v[c0 + i] = t[i];
+                }
             }
             trace_scope.mark(4);
-            const float* part = parts + (size_t)m * Z::PART_LD;   // of rank 0; the others' are MT rows apart
-            auto four = [&](int place) {                          // the sums of four owned columns
-                float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
+            const int first = n0 + rank * OWN;                    // of the columns owned (other than EPI_QKV_ROPE's)
+            if (!ok || !has_token) {
+            } else if (EPI == EPI_SWIGLU) {
+                bf16* out = p.out + (size_t)m * p.ldo + first / 2;
+                uint32_t packed[OWN / 4];
 #pragma unroll
-                for (int o = 0; o < CS; ++o) {
-                    const float4 f = *reinterpret_cast<const float4*>(part + (size_t)o * MT * Z::PART_LD + place);
-                    sum.x += f.x; sum.y += f.y; sum.z += f.z; sum.w += f.w;
-                }
-                return sum;
-            };
-            if (EPI == EPI_SWIGLU) {
-                const int lo = second * (OWN / 2);
-#pragma unroll 1
-                for (int c0 = lo; c0 < lo + OWN / 2; c0 += 16) {
-                    float t[16];
-                    if (CS == 1) {
-                        tmem_16(mine + c0, t);
-                    } else {
+                for (int i = 0; i < OWN / 4; ++i) {
+                    float y[2];
 #pragma unroll
-                        for (int i = 0; i < 16; i += 4) {
-                            const float4 f = four(c0 + i);
-                            t[i] = f.x; t[i + 1] = f.y; t[i + 2] = f.z; t[i + 3] = f.w;
-                        }
+                    for (int e = 0; e < 2; ++e) {
+                        float g = v[4 * i + 2 * e], u = v[4 * i + 2 * e + 1];
+                        if (NORM) { g *= factor; u *= factor; }
+                        if (p.bias) { g += p.bias[first + 4 * i + 2 * e]; u += p.bias[first + 4 * i + 2 * e + 1]; }
+                        // the hardware's base-2 exponent and reciprocal (2^-22 each) for a result that is rounded to bfloat16
+                        float z, r;
+                        asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(z) : "f"(-1.4426950408889634f * g));
+                        asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(1.0f + z));
+                        y[e] = u * (g * r);
                     }
-                    if (!ok || !has_token) continue;
-                    const int first = n0 + rank * OWN + c0;
-                    uint32_t packed[4];
-#pragma unroll
-                    for (int i = 0; i < 4; ++i) {
-                        float y[2];
-#pragma unroll
-                        for (int e = 0; e < 2; ++e) {
-                            float g = t[4 * i + 2 * e], u = t[4 * i + 2 * e + 1];
-                            if (NORM) { g *= factor; u *= factor; }
-                            if (p.bias) { g += p.bias[first + 4 * i + 2 * e]; u += p.bias[first + 4 * i + 2 * e + 1]; }
-                            // the hardware's base-2 exponent and reciprocal (2^-22 each) for a result that is rounded to bfloat16
-                            float z, r;
-                            asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(z) : "f"(-1.4426950408889634f * g));
-                            asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(1.0f + z));
-                            y[e] = u * (g * r);
-                        }
-                        const __nv_bfloat162 h = __floats2bfloat162_rn(y[0], y[1]);
-                        packed[i] = *reinterpret_cast<const uint32_t*>(&h);
-                    }
-                    *reinterpret_cast<uint4*>(p.out + (size_t)m * p.ldo + first / 2) = make_uint4(packed[0], packed[1], packed[2], packed[3]);
+                    const __nv_bfloat162 h = __floats2bfloat162_rn(y[0], y[1]);
+                    packed[i] = *reinterpret_cast<const uint32_t*>(&h);
                 }
+#pragma unroll
+                for (int i = 0; i < OWN / 16; ++i) reinterpret_cast<uint4*>(out)[i] = make_uint4(packed[4 * i], packed[4 * i + 1], packed[4 * i + 2], packed[4 * i + 3]);
             } else if (EPI == EPI_RESID_NORM) {
-                if (ok && resid_mine) {
-                    const int place = OWN > PIECE ? second * PIECE : 0;
-                    const float4 f0 = four(place), f1 = four(place + 4);
-                    float v[PIECE] = {f0.x, f0.y, f0.z, f0.w, f1.x, f1.y, f1.z, f1.w};
-                    const float was[PIECE] = {resid0.x, resid0.y, resid0.z, resid0.w, resid1.x, resid1.y, resid1.z, resid1.w};
-                    const float4 g0 = make_float4(p.gain_out[resid_at], p.gain_out[resid_at + 1], p.gain_out[resid_at + 2], p.gain_out[resid_at + 3]);
-                    const float4 g1 = make_float4(p.gain_out[resid_at + 4], p.gain_out[resid_at + 5], p.gain_out[resid_at + 6], p.gain_out[resid_at + 7]);
-                    const float gain[PIECE] = {g0.x, g0.y, g0.z, g0.w, g1.x, g1.y, g1.z, g1.w};
-                    float sq = 0.f;
-                    uint32_t packed[PIECE / 2];
+                float sq = 0.f;
+                uint32_t packed[OWN / 2];
 #pragma unroll
-                    for (int i = 0; i < PIECE; ++i) {
-                        float y = v[i];
-                        if (NORM) y *= factor;
-                        if (p.bias) y += p.bias[resid_at + i];
-                        v[i] = was[i] + __bfloat162float(__float2bfloat16_rn(y));      // what a stored delta would hold
-                        sq = fmaf(v[i], v[i], sq);
-                    }
-#pragma unroll
-                    for (int i = 0; i < PIECE / 2; ++i) {
-                        const __nv_bfloat162 h = __floats2bfloat162_rn(gain[2 * i] * v[2 * i], gain[2 * i + 1] * v[2 * i + 1]);
-                        packed[i] = *reinterpret_cast<const uint32_t*>(&h);
-                    }
-                    float4* back = reinterpret_cast<float4*>(p.resid_inout + (size_t)m * p.N + resid_at);
-                    back[0] = make_float4(v[0], v[1], v[2], v[3]);
-                    back[1] = make_float4(v[4], v[5], v[6], v[7]);
-                    *reinterpret_cast<uint4*>(p.xn_out + (size_t)m * p.N + resid_at) = make_uint4(packed[0], packed[1], packed[2], packed[3]);
-                    p.ss_out[(size_t)m * (p.N / PIECE) + resid_at / PIECE] = sq;
+                for (int i = 0; i < OWN; ++i) {
+                    float y = v[i];
+                    if (NORM) y *= factor;
+                    if (p.bias) y += p.bias[first + i];
+                    v[i] = resid[i] + __bfloat162float(__float2bfloat16_rn(y));      // what a stored delta would hold
+                    sq = fmaf(v[i], v[i], sq);
                 }
-            } else if (ok && has_token) {                         // EPI_QKV_ROPE: half of the share's pairs a thread
-                const int head = blockIdx.x;
+#pragma unroll
+                for (int i = 0; i < OWN / 2; ++i) {
+                    const __nv_bfloat162 h = __floats2bfloat162_rn(p.gain_out[first + 2 * i] * v[2 * i], p.gain_out[first + 2 * i + 1] * v[2 * i + 1]);
+                    packed[i] = *reinterpret_cast<const uint32_t*>(&h);
+                }
+#pragma unroll
+                for (int i = 0; i < OWN / 4; ++i)
+                    reinterpret_cast<float4*>(p.resid_inout + (size_t)m * p.N + first)[i] = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+#pragma unroll
+                for (int i = 0; i < OWN / 8; ++i)
+                    reinterpret_cast<uint4*>(p.xn_out + (size_t)m * p.N + first)[i] = make_uint4(packed[4 * i], packed[4 * i + 1], packed[4 * i + 2], packed[4 * i + 3]);
+                p.ss_out[(size_t)m * (p.N / OWN) + first / OWN] = sq;
+            } else {                                              // EPI_QKV_ROPE
+                const int head = blockIdx.x, j0 = rank * share;
                 const bool query = head < p.num_heads, key = !query && head < p.num_heads + p.num_kv_heads;
                 bf16* to = nullptr;
                 if (query) {
@@ -334,32 +324,25 @@ batch_kernel(const Params p, const Plan s, const float2* __restrict__ rotations,
                         to = (key ? p.k_cache : p.v_cache) + (slot / p.page_size) * p.page_stride +
                              (long long)(head - p.num_heads - (key ? 0 : p.num_kv_heads)) * p.head_stride + (slot % p.page_size) * BN;
                 }
-                const int lo = second * (share / 2);
-#pragma unroll 1
-                for (int i = lo; i < lo + share / 2; i += 2) {
-                    const int j = rank * share + i;
+#pragma unroll
+                for (int i = 0; i < share; i += 2) {
                     float4 turn = make_float4(1.f, 0.f, 1.f, 0.f);                     // of values: cosine 1, sine 0
-                    if (query || key) turn = __ldcg(reinterpret_cast<const float4*>(rotations + (size_t)m * half + j));
+                    if (query || key) turn = __ldcg(reinterpret_cast<const float4*>(rotations + (size_t)m * half + j0 + i));
                     float x[2][2];
 #pragma unroll
-                    for (int up = 0; up < 2; ++up) {
-                        float2 sum = make_float2(0.f, 0.f);
+                    for (int e = 0; e < 2; ++e)
 #pragma unroll
-                        for (int o = 0; o < CS; ++o) {
-                            const float2 f = *reinterpret_cast<const float2*>(part + (size_t)o * MT * Z::PART_LD + up * share + i);
-                            sum.x += f.x; sum.y += f.y;
+                        for (int up = 0; up < 2; ++up) {
+                            float y = v[up * share + i + e];
+                            if (NORM) y *= factor;
+                            if (p.bias) y += p.bias[head * BN + up * half + j0 + i + e];
+                            x[e][up] = y;
                         }
-                        if (NORM) { sum.x *= factor; sum.y *= factor; }
-                        if (p.bias) {
-                            sum.x += p.bias[head * BN + up * half + j];
-                            sum.y += p.bias[head * BN + up * half + j + 1];
-                        }
-                        x[0][up] = sum.x;
-                        x[1][up] = sum.y;
-                    }
                     if (!to) continue;
-                    *reinterpret_cast<__nv_bfloat162*>(to + j) = __floats2bfloat162_rn(x[0][0] * turn.x - x[0][1] * turn.y, x[1][0] * turn.z - x[1][1] * turn.w);
-                    *reinterpret_cast<__nv_bfloat162*>(to + half + j) = __floats2bfloat162_rn(x[0][0] * turn.y + x[0][1] * turn.x, x[1][0] * turn.w + x[1][1] * turn.z);
+                    *reinterpret_cast<__nv_bfloat162*>(to + j0 + i) =
+                        __floats2bfloat162_rn(x[0][0] * turn.x - x[0][1] * turn.y, x[1][0] * turn.z - x[1][1] * turn.w);
+                    *reinterpret_cast<__nv_bfloat162*>(to + half + j0 + i) =
+                        __floats2bfloat162_rn(x[0][0] * turn.y + x[0][1] * turn.x, x[1][0] * turn.w + x[1][1] * turn.z);
                 }
             }
         }
@@ -446,7 +429,7 @@ EG_API int eg_gemm_batch_takes(int epilogue, int N, int K, int head_dim) {
     batch_plan::Kind kind;
     batch_plan::Cut c{};
     if (!kind_of(epilogue, &kind) || !batch_plan::cut_for(kind, N, K, head_dim, &c)) return 0;
-    return kind == batch_plan::INTO_RESIDUAL ? N / 8 : 1;
+    return kind == batch_plan::INTO_RESIDUAL ? N / (c.columns / c.split) : 1;
 }
 
 // One product of a decode chain for M of 17 to 64 tokens.  epilogue 2 (SwiGLU of interleaved gate and up rows, out [M, N / 2]) and 3 (bias,

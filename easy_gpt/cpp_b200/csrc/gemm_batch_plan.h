@@ -23,7 +23,7 @@ inline bool cut_for(Kind kind, int N, int K, int head_dim, Cut* out) {
     }
     if (N % c.columns) return false;
     const int tiles = N / c.columns, chunks = K / BK;
-    // SwiGLU's tiles are many; the others own 8 or 16 of a tile's columns, QKV's a share of its pairs
+    // SwiGLU's tiles are many; the others own 8 or 16 of a tile's columns, QKV's a share of its pairs in pieces of four at least
     const int least = kind == SWIGLU ? 1 : 4, most = kind == SWIGLU ? 2 : 8;
     c.split = least;
     while (c.split < most && tiles * c.split * 2 <= 2 * SMS && (tiles * c.split < 100 || tiles * c.split * 2 <= SMS) && chunks >= c.split * 4) c.split *= 2;
