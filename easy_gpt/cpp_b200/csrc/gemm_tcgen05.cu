@@ -564,7 +564,8 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
         if (lane == 0) {                                         // ---- TMA producer, in both CTAs
             int g = 0;
             bool ok = true;
-            // the weights of the first tile's first stages are asked for before the kernel in front is known to be done
+            // the weights of the first tile's first stages are asked for before the kernel in front is known to be done (a prompt of
+            // 2,048 tokens at the 0.5B sizes, 24 of these products: 2,718 us started behind it, 2,674 so)
             const int early = min(PSTAGES, k_blocks);
             {
                 const int n0 = (pair / m_tiles) * PBN + rank * (PBN / 2);

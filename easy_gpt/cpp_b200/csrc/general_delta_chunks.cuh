@@ -14,7 +14,8 @@
 //
 // Everything is float32 multiply-adds.  What bounds the chain: 64 x 16 of them a token and 16 columns, 512 cycles a chunk of what an
 // SM can do, and two trips through shared memory (H's parts, the state).  A block has 16 columns of a head: 128 blocks for 32
-// heads and one prompt.  Four warps have the state in registers and work out H and D^T H, four more the outputs and, a chunk
+// heads and one prompt.  (Measured: a prompt of 2,047 tokens through six layers, four of them this rule, 3.61 ms with blocks of four tokens,
+// 3.18 with this.)  Four warps have the state in registers and work out H and D^T H, four more the outputs and, a chunk
 // ahead, K^T V.
 #pragma once
 
