@@ -69,7 +69,7 @@ __global__ void __launch_bounds__(128) general_delta_chunks_kernel(const DeltaPa
         float kk = fmaf(k.x, k.x, fmaf(k.y, k.y, fmaf(k.z, k.z, k.w * k.w)));
 #pragma unroll
         for (int o = 8; o > 0; o >>= 1) kk += __shfl_xor_sync(0xffffffffu, kk, o);
-        const float inv = 1.0f / sqrtf(kk + p.unit_eps);
+        const float inv = live ? 1.0f / sqrtf(kk + p.unit_eps) : 0.f;        // (what fills a chunk up has no key to divide by, whatever unit_eps is)
         auto decay = [&](float z) { return live ? decay_exp(-p.decay_scale * sigmoid_f(z)) : 1.0f; };
         const float4 u = make_float4(k.x * inv, k.y * inv, k.z * inv, k.w * inv);
         *reinterpret_cast<float4*>(&sw[t][d]) = make_float4(decay(x.x + w0.x), decay(x.y + w0.y), decay(x.z + w0.z), decay(x.w + w0.w));

@@ -21,14 +21,14 @@ def problem(counts, heads, dim, rate, seed):
     return p
 
 
-def exact(p, counts, heads, dim):
+def exact(p, counts, heads, dim, unit_eps=UNIT_EPS):
     n = heads * dim
     sig = lambda z: 1 / (1 + np.exp(-z))  # noqa: E731
     q = {k: v.astype(np.float64) for k, v in p.items()}
     r, k, v, g, a = (q["proj"][:, i * n:(i + 1) * n].reshape(-1, heads, dim) for i in range(5))
     w = np.exp(-np.float64(np.float32(SCALE)) * sig(q["x"] + q["w0"])).reshape(-1, heads, dim)
     rate = sig(a + q["a0"].reshape(heads, dim))
-    u = k / np.sqrt((k * k).sum(-1, keepdims=True) + UNIT_EPS)
+    u = k / np.sqrt((k * k).sum(-1, keepdims=True) + unit_eps)
     out, state, at = np.zeros_like(v), np.zeros((len(counts), heads, dim, dim)), 0
     for s, c in enumerate(counts):
         S = q["state"][s].transpose(0, 2, 1).copy()             # the slot keeps [head, column, row]
@@ -41,7 +41,7 @@ def exact(p, counts, heads, dim):
     return y.reshape(-1, n), state
 
 
-def kernel(p, counts, heads, dim, lib=None):
+def kernel(p, counts, heads, dim, lib=None, unit_eps=UNIT_EPS):
     import torch
 
     from easy_gpt.cpp_b200 import kernels
@@ -62,7 +62,7 @@ def kernel(p, counts, heads, dim, lib=None):
     status = torch.zeros(1, dtype=torch.int32, device="cuda")
     rc = fn(torch.cuda.current_stream().cuda_stream, dev["proj"].data_ptr(), dev["proj"].shape[1], 0, n, 2 * n, 3 * n, 4 * n, 5 * n, dev["x"].data_ptr(), n, None, 0, 8,
             dev["w0"].data_ptr(), dev["a0"].data_ptr(), dev["gain"].data_ptr(), records.data_ptr(), state.data_ptr(), n * dim, 0, starts.data_ptr(),
-            slot_ids.data_ptr(), y.data_ptr(), 0, n, o_raw.data_ptr(), 4, T, len(counts), heads, dim, UNIT_EPS, EPS, SCALE, status.data_ptr())
+            slot_ids.data_ptr(), y.data_ptr(), 0, n, o_raw.data_ptr(), 4, T, len(counts), heads, dim, unit_eps, EPS, SCALE, status.data_ptr())
     torch.cuda.synchronize()
     assert rc == 0 and int(status[0]) == 0
     return y.cpu().numpy(), torch.stack([state[s] for s in slots]).reshape(len(counts), heads, dim, dim).cpu().numpy()
@@ -83,3 +83,13 @@ def test_prompts_in_chunks(heads, dim, counts, rate):
     want_y, want_state = exact(p, counts, heads, dim)
     assert np.isfinite(y).all()
     assert off(y, want_y) < 4e-6 and off(state, want_state) < 4e-6, (off(y, want_y), off(state, want_state))
+
+
+@pytest.mark.parametrize("counts", [[33], [32], [47, 17], [5, 90, 16, 48]])
+def test_keys_without_an_epsilon(counts):
+    """unit_eps 0 is a key over its length: what fills up an entry's last chunk has no length, and must not divide by it."""
+    p = problem(counts, 2, 64, 0.0, 77 + counts[0])
+    y, state = kernel(p, counts, 2, 64, unit_eps=0.0)
+    want_y, want_state = exact(p, counts, 2, 64, unit_eps=0.0)
+    assert np.isfinite(y).all() and np.isfinite(state).all()
+    assert off(y, want_y) < 4e-6 and off(state, want_state) < 4e-6
