@@ -844,8 +844,8 @@ public:
             if (plans::gemm_skinny_takes(dtype, T, hidden_) && Linear::aligned(x)) {
                 act = gate_up_.skinny_clamped_glu(ctx, x, limit_);
             } else if (plans::gemm_tcgen05_wide_takes(dtype, T, 2 * inter_, hidden_) && Linear::aligned(x)) {
-                launch_check(eg_gemm_tcgen05_pair_glu_bias(ctx.stream, x.p, x.ld, gate_up_.weight, hidden_, gate_up_.bias_f32(), act.p, inter_, T, 2 * inter_,
-                                                           hidden_, ctx.status, limit_), "gemm_tcgen05_pair_glu");
+                launch_check(eg_gemm_tcgen05_pair_constant(ctx.stream, plans::EPI_SWIGLU, x.p, x.ld, gate_up_.weight, hidden_, gate_up_.bias_f32(), act.p, inter_, T,
+                                                           2 * inter_, hidden_, 256, ctx.status, limit_, 0.f), "gemm_tcgen05_pair_glu");
             } else {
                 // the bare product in float32; biases, limits and the gate in one kernel behind it
                 const Rows gu = gate_up_.without_bias_f32(ctx, x);
@@ -869,8 +869,8 @@ public:
                 gate_up_.skinny(ctx, plans::EPI_SWIGLU, T, &x, nullptr, act.p, inter_, nullptr, nullptr, nullptr, nullptr, nullptr);
             } else if (plans::gemm_tcgen05_wide_takes(dtype, T, 2 * inter_, hidden_) && Linear::aligned(x)) {
                 // prompts: the product on the tcgen05 tensor cores (CTA pairs, 256 x 256 tiles) with SwiGLU in its epilogue
-                launch_check(eg_gemm_tcgen05_pair(ctx.stream, plans::EPI_SWIGLU, x.p, x.ld, gate_up_.weight, hidden_, gate_up_.bias_f32(), act.p, inter_, T,
-                                                  2 * inter_, hidden_, 256, ctx.status, nullptr), "gemm_tcgen05_pair");
+                launch_check(eg_gemm_tcgen05_pair_constant(ctx.stream, plans::EPI_SWIGLU, x.p, x.ld, gate_up_.weight, hidden_, gate_up_.bias_f32(), act.p, inter_, T,
+                                                           2 * inter_, hidden_, 256, ctx.status, 0.f, 0.f), "gemm_tcgen05_pair");
             } else {
                 const Rows gu = gate_up_(ctx, x);
                 launch_check(eg_swiglu(ctx.stream, (int)dtype, gu.p, (int)gu.ld, act.p, inter_, T, inter_), "swiglu");
@@ -928,8 +928,8 @@ public:
         } else if (plans::gemm_tcgen05_wide_takes(dtype, T, ff_, hidden_) && Linear::aligned(h)) {
             // prompts: the product on the tcgen05 tensor cores (CTA pairs) with the activation in its epilogue
             act = Rows{ctx.take_rows(T, ff_, dtype), dtype, T, ff_, ff_};
-            launch_check((gelu_ ? eg_gemm_tcgen05_pair_gelu : eg_gemm_tcgen05_pair_relu2)(ctx.stream, h.p, h.ld, up_.weight, hidden_, act.p, ff_, T, ff_, hidden_,
-                                                                                         256, ctx.status), "gemm_tcgen05_pair_act");
+            launch_check(eg_gemm_tcgen05_pair_constant(ctx.stream, gelu_ ? plans::EPI_GELU : plans::EPI_RELU2, h.p, h.ld, up_.weight, hidden_, nullptr, act.p, ff_, T,
+                                                       ff_, hidden_, 256, ctx.status, 0.f, 0.f), "gemm_tcgen05_pair_act");
         } else {
             act = Rows{ctx.take_rows(T, ff_, dtype), dtype, T, ff_, ff_};
             const Rows z = up_(ctx, h, /*out_f32=*/true);

@@ -313,7 +313,8 @@ public:
         } else if (plans::gemm_tcgen05_wide_takes(dtype, T, ff_, hidden_) && Linear::aligned(h)) {
             act = Rows{ctx.take_rows(T, ff_, dtype), dtype, T, ff_, ff_};
             // prompts: the product on the tcgen05 tensor cores (CTA pairs, 256 x 256 tiles) with the activation in its epilogue
-            launch_check(eg_gemm_tcgen05_pair_xielu(ctx.stream, h.p, h.ld, up_.weight, hidden_, act.p, ff_, T, ff_, hidden_, 256, ctx.status, above_, below_),
+            launch_check(eg_gemm_tcgen05_pair_constant(ctx.stream, plans::EPI_XIELU, h.p, h.ld, up_.weight, hidden_, nullptr, act.p, ff_, T, ff_, hidden_, 256, ctx.status,
+                                                       above_, below_),
                          "gemm_tcgen05_pair_xielu");
         } else {
             act = Rows{ctx.take_rows(T, ff_, dtype), dtype, T, ff_, ff_};

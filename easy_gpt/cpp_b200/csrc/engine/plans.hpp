@@ -30,7 +30,7 @@ inline int use_pdl() {
     }
     return mode;
 }
-enum Epilogue { EPI_STORE = 0, EPI_F32 = 1, EPI_SWIGLU = 2, EPI_QKV_ROPE = 3, EPI_RESID_NORM = 4, EPI_XIELU = 5, EPI_GELU = 7 };
+enum Epilogue { EPI_STORE = 0, EPI_F32 = 1, EPI_SWIGLU = 2, EPI_QKV_ROPE = 3, EPI_RESID_NORM = 4, EPI_XIELU = 5, EPI_RELU2 = 6, EPI_GELU = 7 };
 
 inline int sm_count() {
     static int count = 0;

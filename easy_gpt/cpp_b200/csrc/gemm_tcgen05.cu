@@ -143,6 +143,7 @@ struct Params {
     // EPI_SWIGLU with glu_limit > 0: the clamped gate (glu_fast).  EPI_RELU2 (pair kernel): out = max(z, 0)^2.
     // EPI_GELU (pair and grouped kernels): out = z / 2 (1 + erf(z / sqrt 2))
     float glu_limit = 0.f;
+    bool constant_weights = false;      // (pair kernel) nothing in the stream writes W: it may be read before the kernel in front is done
 };
 
 __global__ void __launch_bounds__(THREADS)
@@ -564,9 +565,10 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
         if (lane == 0) {                                         // ---- TMA producer, in both CTAs
             int g = 0;
             bool ok = true;
-            // the weights of the first tile's first stages are asked for before the kernel in front is known to be done (a prompt of
-            // 2,048 tokens at the 0.5B sizes, 24 of these products: 2,718 us started behind it, 2,674 so)
+            // weights that nothing in the stream writes: the first tile's first stages are asked for before the kernel in front is known to
+            // be done (a prompt of 2,048 tokens at the 0.5B sizes, 24 of these products: 2,718 us started behind it, 2,674 so)
             const int early = min(PSTAGES, k_blocks);
+            if (!p.constant_weights) asm volatile("griddepcontrol.wait;\n" ::: "memory");
             {
                 const int n0 = (pair / m_tiles) * PBN + rank * (PBN / 2);
                 for (int kb = 0; kb < early; ++kb) {
@@ -576,7 +578,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
                     tma_load_2d_pair(w + C::W_SUB_BYTES, &map_w, &full_bar[kb], kb * PBK + BK, n0);
                 }
             }
-            asm volatile("griddepcontrol.wait;\n" ::: "memory");
+            if (p.constant_weights) asm volatile("griddepcontrol.wait;\n" ::: "memory");
             asm volatile("griddepcontrol.launch_dependents;\n" ::);
             for (int t = pair; t < total_tiles && ok; t += pairs) {
                 const int n0 = (t / m_tiles) * PBN + rank * (PBN / 2), m0 = (t % m_tiles) * 2 * BM + rank * BM;
@@ -1159,7 +1161,7 @@ int launch_pair(cudaStream_t stream, const CUtensorMap& map_a, const CUtensorMap
 // K % 64 == 0; epilogues as eg_gemm_tcgen05 (SwiGLU with tile_n 256 only).
 static int gemm_tcgen05_pair_any(cudaStream_t stream, int epilogue, const void* A, long long lda, const void* W, long long ldw,
                                  const float* bias, void* out, long long ldo, int M, int N, int K, int tile_n, int* status,
-                                 long long* trace, float act_a, float act_b) {
+                                 long long* trace, bool constant_weights, float act_a, float act_b) {
     if (M <= 0 || N <= 0) return 0;
     if ((tile_n != 128 && tile_n != 256) || N % tile_n || K % BK || K <= 0 || lda % 8 || ldw % 8 || ldo % 8 || (uintptr_t)A % 16 ||
         (uintptr_t)W % 16 || (uintptr_t)out % 16 || (epilogue != EPI_STORE && epilogue != EPI_SWIGLU && epilogue != EPI_XIELU && epilogue != EPI_RELU2 &&
@@ -1177,49 +1179,28 @@ static int gemm_tcgen05_pair_any(cudaStream_t stream, int epilogue, const void* 
         make_map(&map_out, out, M, epilogue == EPI_SWIGLU ? N / 2 : N, ldo, 32))
         return (int)cudaErrorInvalidValue;
     Params p{(bf16*)out, ldo, bias, M, N, K, epilogue, status, trace};
+    p.constant_weights = constant_weights;
     p.act_a = act_a;
     p.act_b = act_b;
     if (epilogue == EPI_SWIGLU) p.glu_limit = act_a;              // the clamped gate's limit rides in act_a (0: SwiGLU)
     return tile_n == 256 ? launch_pair<256>(stream, map_a, map_w, map_out, p, sm_count) : launch_pair<128>(stream, map_a, map_w, map_out, p, sm_count);
 }
 
+// (W and the bias are read when the kernel in front is done, which may have written them.)
 EG_API int eg_gemm_tcgen05_pair(cudaStream_t stream, int epilogue, const void* A, long long lda, const void* W, long long ldw,
                                 const float* bias, void* out, long long ldo, int M, int N, int K, int tile_n, int* status,
                                 long long* trace) {
     if (epilogue == EPI_XIELU || epilogue == EPI_RELU2 || epilogue == EPI_GELU) return (int)cudaErrorInvalidValue;
-    return gemm_tcgen05_pair_any(stream, epilogue, A, lda, W, ldw, bias, out, ldo, M, N, K, tile_n, status, trace, 0.f, 0.f);
+    return gemm_tcgen05_pair_any(stream, epilogue, A, lda, W, ldw, bias, out, ldo, M, N, K, tile_n, status, trace, false, 0.f, 0.f);
 }
 
-// The same product with the xIELU activation in its epilogue: out = act(A W^T), act(z) = a z^2 + z / 2 for z > 0 and
-// b (e^z - 1 - z) + z / 2 for z <= 0, bfloat16 [M, N].
-EG_API int eg_gemm_tcgen05_pair_xielu(cudaStream_t stream, const void* A, long long lda, const void* W, long long ldw, void* out, long long ldo, int M,
-                                      int N, int K, int tile_n, int* status, float act_a, float act_b) {
-    return gemm_tcgen05_pair_any(stream, EPI_XIELU, A, lda, W, ldw, nullptr, out, ldo, M, N, K, tile_n, status, nullptr, act_a, act_b);
-}
-
-// The same product with a squared ReLU in its epilogue: out = max(A W^T, 0)^2, bfloat16 [M, N].
-EG_API int eg_gemm_tcgen05_pair_relu2(cudaStream_t stream, const void* A, long long lda, const void* W, long long ldw, void* out, long long ldo, int M,
-                                      int N, int K, int tile_n, int* status) {
-    return gemm_tcgen05_pair_any(stream, EPI_RELU2, A, lda, W, ldw, nullptr, out, ldo, M, N, K, tile_n, status, nullptr, 0.f, 0.f);
-}
-
-// The same product with the exact gelu in its epilogue: out = z / 2 (1 + erf(z / sqrt 2)), z = A W^T, bfloat16 [M, N].
-EG_API int eg_gemm_tcgen05_pair_gelu(cudaStream_t stream, const void* A, long long lda, const void* W, long long ldw, void* out, long long ldo, int M,
-                                     int N, int K, int tile_n, int* status) {
-    return gemm_tcgen05_pair_any(stream, EPI_GELU, A, lda, W, ldw, nullptr, out, ldo, M, N, K, tile_n, status, nullptr, 0.f, 0.f);
-}
-
-// The same product over interleaved gate and up columns with the clamped gate in its epilogue, out bfloat16 [M, N / 2]:
-// g = min(gate, limit), u = clamp(up, -limit, limit), out = g sigmoid(1.702 g) (u + 1).  Tiles of 256 x 256.
-EG_API int eg_gemm_tcgen05_pair_glu(cudaStream_t stream, const void* A, long long lda, const void* W, long long ldw, void* out, long long ldo, int M,
-                                    int N, int K, int* status, float limit) {
-    if (!(limit > 0.f)) return (int)cudaErrorInvalidValue;
-    return gemm_tcgen05_pair_any(stream, EPI_SWIGLU, A, lda, W, ldw, nullptr, out, ldo, M, N, K, 256, status, nullptr, limit, 0.f);
-}
-
-// The same with a bias float32 [N] (interleaved like the rows of W) added to the sums in front of the gate.
-EG_API int eg_gemm_tcgen05_pair_glu_bias(cudaStream_t stream, const void* A, long long lda, const void* W, long long ldw, const float* bias, void* out,
-                                         long long ldo, int M, int N, int K, int* status, float limit) {
-    if (!(limit > 0.f)) return (int)cudaErrorInvalidValue;
-    return gemm_tcgen05_pair_any(stream, EPI_SWIGLU, A, lda, W, ldw, bias, out, ldo, M, N, K, 256, status, nullptr, limit, 0.f);
+// The same product of weights and a bias that nothing in the stream writes, a model's: W is read ahead, while the kernel in front still
+// runs.  Further epilogues, bfloat16 out: xIELU [M, N], act(z) = a z^2 + z / 2 for z > 0 and b (e^z - 1 - z) + z / 2 for z <= 0, with
+// a = act_a, b = act_b; the squared ReLU max(z, 0)^2; the exact gelu z / 2 (1 + erf(z / sqrt 2)); and with act_a > 0 the SwiGLU
+// epilogue's gate is the clamped one with that limit: g = min(gate, limit), u = clamp(up, -limit, limit), g sigmoid(1.702 g) (u + 1).
+EG_API int eg_gemm_tcgen05_pair_constant(cudaStream_t stream, int epilogue, const void* A, long long lda, const void* W, long long ldw,
+                                         const float* bias, void* out, long long ldo, int M, int N, int K, int tile_n, int* status, float act_a,
+                                         float act_b) {
+    if (epilogue == EPI_SWIGLU && !(act_a >= 0.f)) return (int)cudaErrorInvalidValue;
+    return gemm_tcgen05_pair_any(stream, epilogue, A, lda, W, ldw, bias, out, ldo, M, N, K, tile_n, status, nullptr, true, act_a, act_b);
 }

@@ -157,3 +157,31 @@ def test_cta_pair_swiglu(M, I, K):
     want = uv * (gv / (1 + torch.exp(-gv)))
     assert status.item() == 0
     assert float((out.float() - want).abs().max()) <= 1e-2 * float(want.abs().max())
+
+
+@pytest.mark.parametrize("swiglu", [False, True])
+def test_cta_pair_product_of_a_weight_that_the_kernel_in_front_writes(swiglu):
+    """The kernel in front lets its dependents start before it writes: the product must not have read any of the weight by then."""
+    import ctypes
+
+    from easy_gpt.cpp_b200 import kernels
+
+    lib, P, L, I = kernels.library(), ctypes.c_void_p, ctypes.c_longlong, ctypes.c_int
+    M, N, K = 512, 4096, 896
+    g = torch.Generator().manual_seed(M)
+    x = bf(torch.randn(M, K, generator=g)).to(DEV)
+    sources = [(torch.randn(N, K, generator=g) * 0.05).to(DEV) for _ in range(4)]
+    w, status = torch.zeros(N, K, dtype=torch.bfloat16, device=DEV), torch.zeros(1, dtype=torch.int32, device=DEV)
+    outs = [torch.empty(M, N // 2 if swiglu else N, dtype=torch.bfloat16, device=DEV) for _ in range(12)]
+    convert = lib.eg_convert_columns
+    convert.argtypes = [P, P, L, P, I, L, I, I, I]
+    for i, out in enumerate(outs):
+        assert convert(torch.cuda.current_stream().cuda_stream, sources[i % 4].data_ptr(), K, w.data_ptr(), 1, K, N, K, K) == 0
+        kernels.gemm_tcgen05(x, w, None, out, status, swiglu_epilogue=swiglu, pair=True)
+    torch.cuda.synchronize()
+    assert status.item() == 0
+    for i, out in enumerate(outs):
+        want = x.float() @ bf(sources[i % 4]).float().t()
+        if swiglu:
+            want = want[:, 1::2] * torch.nn.functional.silu(want[:, 0::2])
+        assert float((out.float() - want).abs().max()) <= 1e-2 * float(want.abs().max()), i
