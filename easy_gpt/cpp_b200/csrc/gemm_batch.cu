@@ -102,7 +102,6 @@ batch_kernel(const Params p, const Plan s, const float2* __restrict__ rotations,
     const int kb0 = s.chunks * rank / CS, k_blocks = s.chunks * (rank + 1) / CS - kb0;
     const int ahead = min(k_blocks, s.stages);
 
-    if (p.use_pdl == 1) asm volatile("griddepcontrol.launch_dependents;\n" ::);
     if (threadIdx.x == 64) {
         for (int i = 0; i < s.stages; ++i) {
             mbar_init(&full[i], 1);
@@ -141,6 +140,8 @@ batch_kernel(const Params p, const Plan s, const float2* __restrict__ rotations,
     }
     asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
     const uint32_t tmem = tmem_slot;
+    // Not before this CTA has its columns of TMEM: a CTA of the kernel behind that took the last of them would wait for this one, and it for them.
+    if (p.use_pdl == 1) asm volatile("griddepcontrol.launch_dependents;\n" ::);
     trace_scope.mark(0);
     if (p.use_pdl) asm volatile("griddepcontrol.wait;\n" ::: "memory");
     trace_scope.mark(1);

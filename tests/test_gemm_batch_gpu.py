@@ -107,3 +107,30 @@ def test_products(epilogue, N, K, heads, M):
     got, want = run(epilogue, M, N, K, np.random.default_rng([epilogue, M, N]), heads, with_bias=(M % 2 == 1))
     for g, w, bound in zip(got, want, (2.0 ** -8, 2.0 ** -8, 1e-6)):
         assert off(g, w) < bound, off(g, w)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("M,N,K", [(32, 64, 256), (64, 896, 896), (17, 2048, 256)])
+def test_a_chain_of_products_whatever_the_dependents_wait_for(M, N, K):
+    """Products one behind the other, started when the one in front is done (0), when it has begun (1) and when it has passed its own
+    wait (2): the same sums, bit for bit."""
+    import torch
+
+    lib, rng = library(), np.random.default_rng([M, N, K])
+    f32 = lambda *s: torch.from_numpy(rng.standard_normal(s).astype(np.float32)).cuda()  # noqa: E731
+    W, x, resid, gain = bf16(rng, N, K).cuda(), bf16(rng, M, K).cuda(), f32(M, N) * 30, f32(N)
+    parts = lib.eg_gemm_batch_takes(RESID, N, K, 0)
+    got = []
+    for mode in (0, 1, 2):
+        r, xn, ss = resid.clone(), torch.empty(M, N, device="cuda", dtype=torch.bfloat16), torch.empty(M, parts, device="cuda")
+        status = torch.zeros(1, dtype=torch.int32, device="cuda")
+        for _ in range(24):
+            assert lib.eg_gemm_batch(torch.cuda.current_stream().cuda_stream, RESID, mode, W.data_ptr(), K, None, M, N, K, x.data_ptr(), K, 1e-6, None, 0, None, 0, 0, 0, 0,
+                                     None, None, None, None, 1, 0, 0, 0, r.data_ptr(), gain.data_ptr(), xn.data_ptr(), ss.data_ptr(), None, 0, status.data_ptr()) == 0
+        torch.cuda.synchronize()
+        assert int(status[0]) == 0
+        got.append((r, xn, ss))
+    step = (x.double() @ W.double().T).float().bfloat16().float()           # (a step's rounding may go the other way where its sum is off by a little)
+    assert off(got[0][0] - resid, 24 * step.double()) < 2.0 ** -8
+    for other in got[1:]:
+        assert all(bool((a == b).all()) for a, b in zip(got[0], other))
