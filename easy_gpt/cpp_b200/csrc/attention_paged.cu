@@ -633,15 +633,32 @@ int launch(cudaStream_t stream, const Params& p, int tokens) {
     // 16 clusters are 112 CTAs and the step takes 1.59 ms with them, 1.45 with 256 four-warp CTAs.
     constexpr int WIDE_KEYS = HD <= 64 ? 32 : 16;                                // keys a warp of the eight-warp form takes of a tile
     const long long most_tiles = ((long long)p.table_stride * p.page_size + TILE_KEYS - 1) / TILE_KEYS;
-    // Short contexts: the eight-warp form takes four tiles of heads of 64 (two of 128) at a time, so a CTA walks a context of 512 in two (four)
-    // rounds by itself, and nothing is merged across CTAs.  Heads of 128 only where the launch has 16 pairs and more: fewer are better
-    // off in two CTAs each.  (us a decode step, two four-warp CTAs / one of eight warps: 0.5B sizes, 300 keys, batch 1 / 8 / 16, 592 / 636 /
-    // 739 and 593 / 630 / 727; up to 1,024 keys, 700 of them, batch 1, 593 and 624; 1.5B sizes, 300 keys, 1,088 / 1,194 / 1,347 and 1,100 /
-    // 1,193 / 1,314.)
-    if constexpr (HD <= 128) if (most_tiles <= 8 && (long long)grid.x * grid.y <= sm_count && (HD <= 64 || grid.x * grid.y >= 16)) {
+    // Short contexts: a CTA walks up to 512 keys by itself, and nothing is merged across CTAs.  Heads of 32 and 64: eight warps take two
+    // key tiles at a time, from three tiles on sixteen warps take four (heads of 32 in large launches eight, which leave room for a second
+    // CTA on an SM).  Heads of 128: eight warps, from 16 (token, KV head) pairs on; fewer are better off in two CTAs each.  A warp takes 16 keys of
+    // a tile, not 32 (up to 10% faster): the largest key that a warp has seen has the weight 1, which bfloat16 holds exactly, and with half as
+    // many such keys the result was off by 2 to 4% more at up to 128 keys and by 1 to 2% more at 512 than with four warps in the launches
+    // of before; so it is off by at most as much, by 2 to 4% less from 100 keys on.
+    // Launches of more than half the SMs find no room beside the kernel in front (a CTA has an SM's shared memory), which costs more than the
+    // form gives up to where the walk is long.
+    // (us a launch one behind the other, four warps / this, at 40, 100, 250, 300, 400, 512 keys in tables of 64, 128, 256, 512, 512, 512: 14 heads of 64
+    // on 2, 8 tokens 2.70 3.17 4.19 4.27 4.78 4.87 / 2.65 2.82 3.59 4.18 4.54 4.78; 36 tokens 2.74 3.25 4.63 5.21 5.80 6.16 / 2.73 2.91 3.72 4.27 4.69
+    // 4.93; 64 tokens 2.82 3.60 5.04 7.61 8.46 9.44 / 4.02 4.27 4.95 5.63 6.24 6.66.  16 heads of 32 on 2, 64 tokens 2.39 2.74 3.76 at up to 250 and 7.08 at
+    // 512 / 2.42 2.56 3.33 and 4.70.  12 heads of 128 on 2, 16 tokens 3.67 4.18 6.18 6.32 7.34 7.35 / 3.59 3.85 4.96 5.72 7.21 7.69; 48 tokens 3.76 4.68
+    // 6.49 8.71 10.05 10.30 / 4.27 4.79 6.28 7.09 8.57 9.05.)
+    const long long pairs = (long long)grid.x * grid.y;
+    if constexpr (HD <= 128) if (most_tiles <= 8 && pairs <= sm_count) {
+        const bool small = 2 * pairs <= sm_count;
         Params whole = p;
         whole.splits = 1;
-        return launch_with<HD, true, MASKED, 2, WIDE_KEYS>(stream, whole, dim3(grid.x, grid.y, 1));
+        const dim3 one(grid.x, grid.y, 1);
+        if constexpr (HD == 128) {
+            if (small ? pairs >= 16 : most_tiles >= 6) return launch_with<HD, true, MASKED, 2, 16>(stream, whole, one);
+        } else if (small ? most_tiles <= 2 : HD == 32) {
+            return launch_with<HD, true, MASKED, 2, 16>(stream, whole, one);
+        } else if (small || most_tiles >= 6) {
+            return launch_with<HD, false, MASKED, 4, 16>(stream, whole, one);
+        }
     }
     if constexpr (HD <= 128) if (ctas <= 2ll * sm_count && p.splits >= 4 && p.splits % 2 == 0) {
         for (int fewer = 0; fewer <= 2; ++fewer) {
