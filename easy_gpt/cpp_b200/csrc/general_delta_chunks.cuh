@@ -1,5 +1,5 @@
 // The generalised delta rule (general_delta.cu) over prompts, heads of 64: tokens in chunks of 16 (counted from the entry's first
-// token of the step; the last one is filled up with tokens that change nothing).
+// token of the step; the last one is filled up in front with tokens that change nothing).
 //
 // With G_t = w_0 .. w_t channel by channel and S the state in front of a chunk, what the tokens' old states hold along their unit
 // keys, H (a row h_t per token), satisfies (1 + A) H = U S + B V, where A and B are strictly lower triangular,
@@ -12,11 +12,18 @@
 // (1 + A) H0 = B V by forward substitution, R - Q X and P V - Q H0.  What is left in the chain of chunks is
 //   H = X S + H0;   O = (R - Q X) S + (P V - Q H0);   S' = diag(G_15) S + K^T V - D^T H.
 //
-// Everything is float32 multiply-adds.  What bounds the chain: 64 x 16 of them a token and 16 columns, 512 cycles a chunk of what an
-// SM can do, and two trips through shared memory (H's parts, the state).  A block has 16 columns of a head: 128 blocks for 32
-// heads and one prompt.  (Measured: a prompt of 2,047 tokens through six layers, four of them this rule, 3.61 ms with blocks of four tokens,
-// 3.18 with this.)  Four warps have the state in registers and work out H and D^T H, four more the outputs and, a chunk
-// ahead, K^T V.
+// Sums are float32; the running products of the decays are worked out in 64 bits and rounded once.  Where two kinds of terms meet (what
+// tokens write and what they take off) each kind is added up by itself, and S gets their sum in one step: added onto S one after the
+// other, sixteen roundings of S's size a chunk, the state was twice as far off the result in 64 bits as block by block.  The last term of
+// K^T V is added exactly (the loss goes along): with fast decays it is most of the sum.  (2-norm errors x 1e-8 of the state and of the gated
+// outputs, blocks of four / this, by the mean logit of the decays, 257 tokens: -9, 28.2 24.5 / 20.2 19.9; -2, 9.4 14.2 / 8.8 14.1; 0, 7.1 13.8 / 6.6
+// 13.2; 5, 5.7 15.5 / 5.0 12.8.)
+//
+// What bounds the chain: its latency, two trips through shared memory a chunk (H's parts, the state) with two barriers of four warps and
+// one of eight.  A chunk is 1.25 us, about 2,400 cycles; the multiply-adds of its four products, 64 x 16 a token and 16 columns each, are 512 of
+// them.  A block has 16 columns of a head: 128 blocks for 32 heads and one prompt.  (Measured: the rule over 2,047 tokens, 32 heads, 357 us with
+// blocks of four tokens, 253 with this; 8 entries of 256 tokens 248 and 213.)  Four warps have the state in registers and work out H and
+// D^T H, four more the outputs and, a chunk ahead, K^T V.
 #pragma once
 
 constexpr int CHUNK = 16, CHUNK_DIM = 64, CHUNK_COLS = 16;
@@ -61,11 +68,12 @@ __global__ void __launch_bounds__(128) general_delta_chunks_kernel(const DeltaPa
 #pragma unroll
     for (int half = 0; half < 2; ++half) {
         const int t = (tid >> 4) + half * 8;
-        const bool live = t < count;
+        const bool live = t >= CHUNK - count;
+        const int token = live ? first + t - (CHUNK - count) : first;
         const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
-        const float* row = p.proj + (size_t)(first + (live ? t : 0)) * p.ldp + at + d;
+        const float* row = p.proj + (size_t)token * p.ldp + at + d;
         const float4 k = live ? load(row + p.k_col) : zero, r = live ? load(row + p.r_col) : zero, v = live ? load(row + p.v_col) : zero;
-        const float4 a = load(row + p.a_col), x = load(p.x + (size_t)(first + (live ? t : 0)) * p.ldx + at + d);
+        const float4 a = load(row + p.a_col), x = load(p.x + (size_t)token * p.ldx + at + d);
         float kk = fmaf(k.x, k.x, fmaf(k.y, k.y, fmaf(k.z, k.z, k.w * k.w)));
 #pragma unroll
         for (int o = 8; o > 0; o >>= 1) kk += __shfl_xor_sync(0xffffffffu, kk, o);
@@ -135,8 +143,10 @@ __global__ void __launch_bounds__(128) general_delta_chunks_kernel(const DeltaPa
         for (int t = 0; t < CHUNK; ++t) {
             x[t] = (float)(su[t][c] * run);
             run *= sw[t][c];
+            float off = 0.f;
 #pragma unroll
-            for (int j = 0; j < t; ++j) x[t] = fmaf(-coef[0][t][j], x[j], x[t]);
+            for (int j = 0; j < t; ++j) off = fmaf(-coef[0][t][j], x[j], off);
+            x[t] += off;
         }
 #pragma unroll
         for (int t = 0; t < CHUNK; t += 4) *reinterpret_cast<float4*>(rec + c * CHUNK + t) = make_float4(x[t], x[t + 1], x[t + 2], x[t + 3]);
@@ -147,9 +157,10 @@ __global__ void __launch_bounds__(128) general_delta_chunks_kernel(const DeltaPa
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
                 run *= sw[t + e][c];
-                o[e] = (float)(sr[t + e][c] * run);
+                float off = 0.f;
 #pragma unroll
-                for (int j = 0; j <= t + e; ++j) o[e] = fmaf(-coef[3][t + e][j], x[j], o[e]);
+                for (int j = 0; j <= t + e; ++j) off = fmaf(-coef[3][t + e][j], x[j], off);
+                o[e] = (float)(sr[t + e][c] * run) + off;
             }
             *reinterpret_cast<float4*>(rec + CHUNK * CHUNK_DIM + c * CHUNK + t) = make_float4(o[0], o[1], o[2], o[3]);
         }
@@ -169,24 +180,34 @@ __global__ void __launch_bounds__(128) general_delta_chunks_kernel(const DeltaPa
 #pragma unroll
         for (int t = 0; t < CHUNK; ++t) {
             v[t] = sv[t][c];
-            h[t] = 0.f;
+            float in = 0.f, off = 0.f;
 #pragma unroll
-            for (int j = 0; j < t; ++j) h[t] = fmaf(coef[1][t][j], v[j], h[t]);
+            for (int j = 0; j < t; ++j) in = fmaf(coef[1][t][j], v[j], in);
 #pragma unroll
-            for (int j = 0; j < t; ++j) h[t] = fmaf(-coef[0][t][j], h[j], h[t]);
+            for (int j = 0; j < t; ++j) off = fmaf(-coef[0][t][j], h[j], off);
+            h[t] = in + off;
             slice[t * CHUNK_COLS] = v[t];
             slice[(CHUNK + t) * CHUNK_COLS] = h[t];
         }
 #pragma unroll
         for (int t = 0; t < CHUNK; ++t) {
-            float o = 0.f;
+            float in = 0.f, off = 0.f;
 #pragma unroll
-            for (int j = 0; j <= t; ++j) o = fmaf(-coef[3][t][j], h[j], fmaf(coef[2][t][j], v[j], o));
-            slice[(2 * CHUNK + t) * CHUNK_COLS] = o;
+            for (int j = 0; j <= t; ++j) {
+                in = fmaf(coef[2][t][j], v[j], in);
+                off = fmaf(-coef[3][t][j], h[j], off);
+            }
+            slice[(2 * CHUNK + t) * CHUNK_COLS] = in + off;
         }
     }
 }
 
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
+    uint64_t d;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ uint64_t minus(uint64_t v) { return v ^ 0x8000000080000000ull; }
 __device__ __forceinline__ void chunk_bar(int id) { asm volatile("bar.sync %0, 128;\n" ::"r"(id) : "memory"); }
 
 // The chain: a block per (head, entry, 16 columns), 256 threads.
@@ -198,7 +219,7 @@ __global__ void __launch_bounds__(256, 2) general_delta_chain_kernel(const Delta
     __shared__ __align__(16) float state2[2][CHUNK_DIM][CHUNK_COLS * 2];           // the state in front of a chunk, every value twice
     __shared__ __align__(16) float part[2][4][CHUNK][PART_LD];                     // of H and O: four parts of the 64 channels
     __shared__ __align__(16) float off2[CHUNK][CHUNK_COLS * 2];                    // -H, every value twice
-    __shared__ __align__(16) float4 taken[2][2][128];                              // K^T V, a thread's eight values
+    __shared__ __align__(16) float4 taken[2][2][128];                              // K^T V without its last term, a thread's eight values
     const int head = blockIdx.x, seq = blockIdx.y, j0 = blockIdx.z * CHUNK_COLS, tid = threadIdx.x & 127;
     const bool keeper = threadIdx.x < 128;                                          // of the state
     const int start = p.seq_starts[seq], count = p.seq_starts[seq + 1] - start, chunks = (count + CHUNK - 1) / CHUNK;
@@ -249,16 +270,27 @@ __global__ void __launch_bounds__(256, 2) general_delta_chain_kernel(const Delta
     }
     // [16 tokens][16 columns] = m^T state, this warp's quarter of the channels, into part[which]
     auto product = [&](const float* m, const float (*st)[CHUNK_COLS * 2], int which) {
-        uint64_t acc[2][2] = {};
+        // (two sums side by side, of the even and of the odd channels: shorter chains, fewer roundings)
+        uint64_t acc[2][2] = {}, odd[2][2] = {};
         const float* mk = m + quarter * 16 * CHUNK + token;
         const float* sk = &st[quarter * 16][token_col * 2];
 #pragma unroll
-        for (int k = 0; k < 16; ++k) {
+        for (int k = 0; k < 16; k += 2) {
             const ulonglong2 a = *reinterpret_cast<const ulonglong2*>(mk + k * CHUNK), b = *reinterpret_cast<const ulonglong2*>(sk + k * CHUNK_COLS * 2);
             acc[0][0] = fma2(a.x, b.x, acc[0][0]);
             acc[0][1] = fma2(a.y, b.x, acc[0][1]);
             acc[1][0] = fma2(a.x, b.y, acc[1][0]);
             acc[1][1] = fma2(a.y, b.y, acc[1][1]);
+            const ulonglong2 c = *reinterpret_cast<const ulonglong2*>(mk + (k + 1) * CHUNK), d = *reinterpret_cast<const ulonglong2*>(sk + (k + 1) * CHUNK_COLS * 2);
+            odd[0][0] = fma2(c.x, d.x, odd[0][0]);
+            odd[0][1] = fma2(c.y, d.x, odd[0][1]);
+            odd[1][0] = fma2(c.x, d.y, odd[1][0]);
+            odd[1][1] = fma2(c.y, d.y, odd[1][1]);
+        }
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            acc[0][i] = add2(acc[0][i], odd[0][i]);
+            acc[1][i] = add2(acc[1][i], odd[1][i]);
         }
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
@@ -277,11 +309,11 @@ __global__ void __launch_bounds__(256, 2) general_delta_chain_kernel(const Delta
         const float2 z = *reinterpret_cast<const float2*>(plus + sum_token * CHUNK_COLS + sum_col);
         return make_float2((q[0].x + q[1].x) + (q[2].x + q[3].x) + z.x, (q[0].y + q[1].y) + (q[2].y + q[3].y) + z.y);
     };
-    auto take_in = [&](int c) {                                                     // K^T V of chunk c
+    auto take_in = [&](int c) {                                                     // K^T V of chunk c, without its last term
         const float *K = stage_of(c) + 3 * CHUNK * CHUNK_DIM + row, *V = stage_of(c) + CHUNK_SHARED + col;
         uint64_t acc[2][2] = {};
 #pragma unroll
-        for (int j = 0; j < CHUNK; ++j) {
+        for (int j = 0; j < CHUNK - 1; ++j) {
             const ulonglong2 k = *reinterpret_cast<const ulonglong2*>(K + j * CHUNK_DIM);
             const float2 v = *reinterpret_cast<const float2*>(V + j * CHUNK_COLS);
             const uint64_t v0 = pair_of(v.x, v.x), v1 = pair_of(v.y, v.y);
@@ -312,28 +344,49 @@ __global__ void __launch_bounds__(256, 2) general_delta_chain_kernel(const Delta
             const float2 h = sums(0, stage + CHUNK_SHARED + CHUNK * CHUNK_COLS);
             *reinterpret_cast<float4*>(&off2[sum_token][sum_col * 2]) = make_float4(-h.x, -h.x, -h.y, -h.y);
             const ulonglong2 g = *reinterpret_cast<const ulonglong2*>(stage + 4 * CHUNK * CHUNK_DIM + row);
-            const ulonglong2 t0 = *reinterpret_cast<const ulonglong2*>(&taken[c & 1][0][tid]), t1 = *reinterpret_cast<const ulonglong2*>(&taken[c & 1][1][tid]);
-            s[0][0] = fma2(g.x, s[0][0], t0.x);
-            s[0][1] = fma2(g.y, s[0][1], t0.y);
-            s[1][0] = fma2(g.x, s[1][0], t1.x);
-            s[1][1] = fma2(g.y, s[1][1], t1.y);
+            // K^T V's last term, with what its product and its addition lose (an exact product by a fused multiply-add and Knuth's exact sum): -D^T H
+            // is added up from there on
+            ulonglong2 in[2], sum[2];
+            {
+                const ulonglong2 k = *reinterpret_cast<const ulonglong2*>(stage + 3 * CHUNK * CHUNK_DIM + (CHUNK - 1) * CHUNK_DIM + row);
+                const float2 v = *reinterpret_cast<const float2*>(stage + CHUNK_SHARED + (CHUNK - 1) * CHUNK_COLS + col);
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    const ulonglong2 before = *reinterpret_cast<const ulonglong2*>(&taken[c & 1][e][tid]);
+                    const uint64_t b = e ? pair_of(v.y, v.y) : pair_of(v.x, v.x);
+                    auto last = [&](uint64_t a, uint64_t s, uint64_t* lost) {
+                        const uint64_t p = mul2(a, b), t = add2(s, p), z = add2(t, minus(s));
+                        *lost = add2(add2(add2(s, minus(add2(t, minus(z)))), add2(p, minus(z))), fma2(a, b, minus(p)));
+                        return t;
+                    };
+                    uint64_t l0, l1;
+                    in[e].x = last(k.x, before.x, &l0);
+                    in[e].y = last(k.y, before.y, &l1);
+                    sum[e] = make_ulonglong2(l0, l1);
+                }
+            }
             chunk_bar(1);
             const float* D = stage + 2 * CHUNK * CHUNK_DIM + row;
 #pragma unroll
             for (int j = 0; j < CHUNK; ++j) {
                 const ulonglong2 a = *reinterpret_cast<const ulonglong2*>(D + j * CHUNK_DIM), h2 = *reinterpret_cast<const ulonglong2*>(&off2[j][col * 2]);
-                s[0][0] = fma2(a.x, h2.x, s[0][0]);
-                s[0][1] = fma2(a.y, h2.x, s[0][1]);
-                s[1][0] = fma2(a.x, h2.y, s[1][0]);
-                s[1][1] = fma2(a.y, h2.y, s[1][1]);
+                sum[0].x = fma2(a.x, h2.x, sum[0].x);
+                sum[0].y = fma2(a.y, h2.x, sum[0].y);
+                sum[1].x = fma2(a.x, h2.y, sum[1].x);
+                sum[1].y = fma2(a.y, h2.y, sum[1].y);
+            }
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                s[e][0] = fma2(g.x, s[e][0], add2(in[e].x, sum[e].x));
+                s[e][1] = fma2(g.y, s[e][1], add2(in[e].y, sum[e].y));
             }
             put_state((c + 1) & 1);
         } else {
             product(stage + CHUNK * CHUNK_DIM, state2[c & 1], 1);
             chunk_bar(2);
             const float2 o = sums(1, stage + CHUNK_SHARED + 2 * CHUNK * CHUNK_COLS);
-            const int t = c * CHUNK + sum_token;
-            if (ok && t < count)
+            const int skip = c + 1 < chunks ? 0 : chunks * CHUNK - count, t = c * CHUNK + sum_token - skip;
+            if (ok && sum_token >= skip)
                 *reinterpret_cast<float2*>(p.o_raw + (size_t)(start + t) * ((size_t)p.heads * CHUNK_DIM) + head * CHUNK_DIM + j0 + sum_col) = o;
             if (c + 1 < chunks) {
                 ok = arrived(c + 1) && ok;

@@ -93,3 +93,20 @@ def test_keys_without_an_epsilon(counts):
     want_y, want_state = exact(p, counts, 2, 64, unit_eps=0.0)
     assert np.isfinite(y).all() and np.isfinite(state).all()
     assert off(y, want_y) < 4e-6 and off(state, want_state) < 4e-6
+
+
+@pytest.mark.parametrize("rate, of_state, of_outputs", [(-9.0, 2.8e-7, 2.5e-7), (0.0, 8.8e-8, 1.5e-7), (5.0, 7.0e-8, 1.6e-7)])
+@pytest.mark.parametrize("counts", [[257], [64], [40, 200]])
+def test_errors_of_the_chunks(counts, rate, of_state, of_outputs):
+    """A token at a time, S is rounded three times a token (2^-24 / sqrt(3) of its size each), and decays w forget: sqrt(3 / (1 - w^2)) of these at
+    0 and 5.  The chunks are held to that; at -9, where nothing is forgotten, to what blocks of four tokens show (2.8e-7 at 257 tokens), and the
+    outputs, which have roundings of their own (norm and gate), to what those show."""
+    off_state, off_outputs = [], []
+    for seed in range(4):
+        p = problem(counts, 2, 64, rate, 100 + seed)
+        y, state = kernel(p, counts, 2, 64)
+        want_y, want_state = exact(p, counts, 2, 64)
+        off_state.append(off(state, want_state))
+        off_outputs.append(off(y, want_y))
+    rms = lambda e: float(np.sqrt(np.mean(np.square(e))))  # noqa: E731
+    assert rms(off_state) < of_state and rms(off_outputs) < of_outputs, (rms(off_state), rms(off_outputs))
