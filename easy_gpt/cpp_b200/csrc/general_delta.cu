@@ -33,7 +33,8 @@
 // (Prompts through heads of 64 go in chunks of 16 tokens: general_delta_chunks.cuh.)
 //
 // Tiles arrive three stages ahead.  Outputs are normed and gated by the block where it holds a whole head, else by a kernel behind.
-// The slot keeps S as [head, column, row].  The order of every sum depends on the sizes and on a token's place in its block.
+// The slot keeps S as [head, column, row].  The order of every sum depends on the sizes and on a token's place in its block or chunk; for heads
+// of 64 also on the step's tokens and entries, which decide for blocks or chunks (chunks_take).
 #include <algorithm>
 #include <cstdlib>
 
@@ -632,15 +633,23 @@ int dispatch_general_delta(cudaStream_t stream, const DeltaParams& p, int slices
 
 #include "general_delta_chunks.cuh"
 
-// Which prompts go through the chain of chunks: heads of 64, entries of 32 tokens on average.
-bool chunks_take(int tokens, int num_seqs, int dim) { return dim == CHUNK_DIM && tokens >= 2 * CHUNK * num_seqs; }
+// Which steps go through the chain of chunks: heads of 64, entries of 32 tokens on average (the scratch memory holds their chunks), one of which
+// has 48 where there are more than two.  An entry's last chunk is filled up, and every entry has one.  (us of the rule, 32 heads, blocks of
+// four / chunks, entries x tokens: 1 x 32, 20 / 15; 2 x 33, 23.4 / 21.9; 4 x 33, 30.2 / 33.7; 8 x 33, 44.2 / 48.1; 31 x 33, 134 / 171; 4 x 40, 33.0 / 33.8;
+// 4 x 48, 35.6 / 35.8; 8 x 48, 53.6 / 48.5; 31 x 48, 184 / 175; 31 x 64, 231 / 223; 16 x 100, 190 / 190; 31 x 100, 357 / 363; 16 x 256, 448 / 414.  A prompt
+// beside single tokens: 250 and 7 of them, 71 / 61; 500 and 14, 195 / 115; 1,000 and 30, 391 / 242.)
+bool chunks_take(int tokens, int num_seqs, int longest, int dim) {
+    return dim == CHUNK_DIM && tokens >= 2LL * CHUNK * num_seqs && (num_seqs <= 2 || longest >= 3 * CHUNK);
+}
+// the chunks of a step's entries, at most: each entry's tokens / 16, rounded up
+int most_chunks_of(int tokens, int num_seqs) { return (int)((tokens + (CHUNK - 1LL) * num_seqs) / CHUNK); }
 
 template <typename TO>
 int launch_chunks(cudaStream_t stream, DeltaParams p, int num_seqs, bool wide) {
     constexpr int smem = CHUNK_STAGES * CHUNK_STAGE * 4;
     static const cudaError_t configured = cudaFuncSetAttribute(general_delta_chain_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (configured != cudaSuccess) return (int)configured;
-    const int most_chunks = p.tokens / CHUNK + num_seqs;
+    const int most_chunks = most_chunks_of(p.tokens, num_seqs);
     const unsigned blocks = (unsigned)((long long)most_chunks * p.heads);
     if (wide) eg_pdl_launch(general_delta_chunks_kernel<true>, blocks, 128, 0, stream, p, num_seqs, most_chunks);
     else eg_pdl_launch(general_delta_chunks_kernel<false>, blocks, 128, 0, stream, p, num_seqs, most_chunks);
@@ -661,10 +670,15 @@ __global__ void tanh_columns_kernel(const float* __restrict__ src, long long lds
 }
 }  // namespace
 
-// float32 values of scratch memory (`records`) a token and head of `dim` channels: a record, or a token's share of the chunks, of which
-// there are at most tokens / 16 + num_seqs <= 3 tokens / 32
+// Whether a step, whose longest entry has `longest` tokens, goes through the chain of chunks (where the rule has x and o_raw)
+EG_API int eg_general_delta_in_chunks(int tokens, int num_seqs, int longest, int dim) {
+    return tokens > 0 && num_seqs > 0 && chunks_take(tokens, num_seqs, longest, dim);
+}
+
+// float32 values of scratch memory (`records`) a token and head of `dim` channels: a record, or a token's share of the chunks, of which a
+// step has at most (tokens + 15 entries) / 16 <= 47 tokens / (16 x 32)
 EG_API int eg_general_delta_record(int dim) {
-    if (dim == CHUNK_DIM) return std::max(VECS * 64 + NUMBERS, (3 * CHUNK_RECORD / 32 + 3) / 4 * 4);
+    if (dim == CHUNK_DIM) return std::max(VECS * 64 + NUMBERS, (47 * CHUNK_RECORD / (16 * 32) + 4) / 4 * 4);
     return VECS * (dim <= 16 ? 16 : dim <= 32 ? 32 : dim <= 64 ? 64 : dim <= 128 ? 128 : 256) + NUMBERS;
 }
 
@@ -676,12 +690,13 @@ EG_API int eg_general_delta_inline_takes(int entry_tokens, int rank) { return en
 // (w0 still to be added), or null in steps whose entries eg_general_delta_inline_takes: then w2 [heads * dim, ld2] in y_dtype (ld2 a
 // multiple of 8).  a0, w0, gain float32 [heads * dim].  records: scratch, not read with x null.  state: the requests' slots; S of
 // a request lies state_offset floats into its slot.  y [tokens, ldy] in y_dtype.  slices > 1 (with o_raw float32 [tokens, heads * dim]): a
-// head's columns are dealt to that many blocks, and the outputs are normed by a kernel behind.  dim up to 256.
-EG_API int eg_general_delta(cudaStream_t stream, const float* proj, long long ldp, int r_col, int k_col, int v_col, int g_col, int a_col, int inner_col,
-                            const float* x, long long ldx, const void* w2, int ld2, int rank, const float* w0, const float* a0, const float* gain,
-                            float* records, float* state, long long slot_floats, long long state_offset, const int* seq_starts, const int* seq_slots,
-                            void* y, int y_dtype, long long ldy, float* o_raw, int slices, int tokens, int num_seqs, int heads, int dim, float unit_eps,
-                            float eps, float decay_scale, int* status) {
+// head's columns are dealt to that many blocks, and the outputs are normed by a kernel behind.  dim up to 256.  longest: the tokens of
+// the step's longest entry.
+EG_API int eg_general_delta_step(cudaStream_t stream, const float* proj, long long ldp, int r_col, int k_col, int v_col, int g_col, int a_col, int inner_col,
+                                 const float* x, long long ldx, const void* w2, int ld2, int rank, const float* w0, const float* a0, const float* gain,
+                                 float* records, float* state, long long slot_floats, long long state_offset, const int* seq_starts, const int* seq_slots,
+                                 void* y, int y_dtype, long long ldy, float* o_raw, int slices, int tokens, int num_seqs, int heads, int dim, float unit_eps,
+                                 float eps, float decay_scale, int longest, int* status) {
     if (num_seqs <= 0 || tokens <= 0) return 0;
     if (heads <= 0 || dim <= 0 || dim > 256 || slices < 1 || (x && !records) || (!x && (!w2 || ld2 % 8 || (uintptr_t)w2 % 16))) return (int)cudaErrorInvalidValue;
     if (slot_floats % 4 || state_offset % 4 || (uintptr_t)state % 16 || (uintptr_t)records % 16) {
@@ -723,11 +738,22 @@ EG_API int eg_general_delta(cudaStream_t stream, const float* proj, long long ld
     auto aligned = [](const void* q) { return (uintptr_t)q % 16 == 0; };
     const bool wide = ldp % 4 == 0 && ldx % 4 == 0 && r_col % 4 == 0 && k_col % 4 == 0 && v_col % 4 == 0 && g_col % 4 == 0 && a_col % 4 == 0 && aligned(proj) &&
                       aligned(x) && aligned(w0) && aligned(a0) && aligned(gain) && aligned(o_raw) && aligned(y) && ldy % 4 == 0;
-    if (x && o_raw && (uintptr_t)o_raw % 8 == 0 && chunks_take(tokens, num_seqs, dim))
+    if (x && o_raw && (uintptr_t)o_raw % 8 == 0 && chunks_take(tokens, num_seqs, longest, dim))
         return y_dtype == EG_BF16 ? launch_chunks<bf16>(stream, p, num_seqs, wide) : launch_chunks<float>(stream, p, num_seqs, wide);
     if (y_dtype == EG_BF16)
         return x ? dispatch_general_delta<bf16, false>(stream, p, slices, num_seqs, wide) : dispatch_general_delta<bf16, true>(stream, p, slices, num_seqs, wide);
     return x ? dispatch_general_delta<float, false>(stream, p, slices, num_seqs, wide) : dispatch_general_delta<float, true>(stream, p, slices, num_seqs, wide);
+}
+
+// The same where nothing is known of the longest entry
+EG_API int eg_general_delta(cudaStream_t stream, const float* proj, long long ldp, int r_col, int k_col, int v_col, int g_col, int a_col, int inner_col,
+                            const float* x, long long ldx, const void* w2, int ld2, int rank, const float* w0, const float* a0, const float* gain,
+                            float* records, float* state, long long slot_floats, long long state_offset, const int* seq_starts, const int* seq_slots,
+                            void* y, int y_dtype, long long ldy, float* o_raw, int slices, int tokens, int num_seqs, int heads, int dim, float unit_eps,
+                            float eps, float decay_scale, int* status) {
+    return eg_general_delta_step(stream, proj, ldp, r_col, k_col, v_col, g_col, a_col, inner_col, x, ldx, w2, ld2, rank, w0, a0, gain, records, state, slot_floats,
+                                 state_offset, seq_starts, seq_slots, y, y_dtype, ldy, o_raw, slices, tokens, num_seqs, heads, dim, unit_eps, eps, decay_scale,
+                                 tokens - num_seqs + 1, status);
 }
 
 // dst [rows, ldd] in dst_dtype: column c < cols holds tanh(src[., c]), columns up to `padded` hold zeros

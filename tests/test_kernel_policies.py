@@ -93,3 +93,22 @@ def test_no_more_is_asked_ahead_of_the_l2_than_it_can_hold():
 
     for bytes_, want in ((0, 0), (17 << 20, 17 << 20), (32 << 20, 32 << 20), (55 << 20, 32 << 20), (126 << 20, 32 << 20), (37888 * 3584 * 2, 0), (1 << 40, 0)):
         assert native.plan(5, bytes_)[0] == want, bytes_
+
+
+def test_general_delta_steps_in_chunks():
+    """Entries of 32 tokens on average, one of which has 48 where there are more than two (heads of 64): shorter ones are faster in blocks.  The
+    scratch memory that a caller makes from tokens and heads alone holds every such step's chunks: tokens / 16 of each entry, rounded up, of 7,232
+    values each."""
+    from easy_gpt.cpp_b200 import kernels
+
+    lib = kernels.library()
+    takes, record = lib.eg_general_delta_in_chunks, lib.eg_general_delta_record
+    for counts, want in (([31], 0), ([32], 1), ([2047], 1), ([63], 1), ([40, 20], 0), ([33] * 2, 1), ([33] * 3, 0), ([33] * 8, 0), ([33] * 31, 0), ([40] * 4, 0), ([48] * 4, 1),
+                         ([48] * 31, 1), ([500] + [1] * 14, 1), ([1000] + [1] * 30, 1), ([1000] + [1] * 40, 0), ([90, 31, 20, 1], 1)):
+        assert takes(sum(counts), len(counts), max(counts), 64) == want, counts
+    assert not any(takes(4096, 1, 4096, dim) for dim in (16, 32, 63, 65, 128)) and takes(0, 0, 0, 64) == 0
+    for entries in range(1, 80):
+        for tokens in range(entries, 40 * entries + 400):
+            if takes(tokens, entries, tokens - entries + 1, 64):
+                assert (tokens + 15 * entries) // 16 * 7232 <= tokens * record(64)
+    assert record(64) >= 6 * 64 + 8 and record(32) == 6 * 32 + 8
