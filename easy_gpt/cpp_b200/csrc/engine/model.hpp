@@ -25,7 +25,7 @@ struct SubLayer {
     bool plain_pre_norm = false;        // x = x + part(norm(x)) with nothing behind the part: the shape whose add and norm the parts may fuse
     // whether the sub-layer in front may prepare this one's norm: the part must take a norm that is not computed yet
     bool takes_prepared_norm() const { return plain_pre_norm && (mixer ? mixer->accepts_pending_norm() : feed_forward->accepts_pending_norm()); }
-    // the same in steps of 17 to 64 tokens
+    // the same in steps that plans::batch_step takes
     bool takes_prepared_batch(bool writes) const { return takes_prepared_norm() && (mixer ? mixer->takes_prepared_batch(writes) : feed_forward->takes_prepared_batch()); }
     Part* part() const { return mixer ? static_cast<Part*>(mixer.get()) : static_cast<Part*>(feed_forward.get()); }
     std::vector<Part*> parts() const {
@@ -250,7 +250,7 @@ public:
                 FollowingNorm follow;
                 const FollowingNorm* offer = nullptr;
                 const bool fuses = sub.mixer ? sub.mixer->fuses_following_norm() : sub.feed_forward->fuses_following_norm();
-                const bool batch = T > fused_rows && plans::batch_tokens(ctx.dtype, T) &&
+                const bool batch = T > fused_rows && plans::batch_step(ctx.dtype, T, sub.norm->size(), ctx.all_decode) &&
                                    (i + 1 < sublayers.size() ? sublayers[i + 1].takes_prepared_batch(cache.writes) : next_takes_batch);
                 if (fuses && following && following->rms_parameters(&follow.gain, &follow.eps) && ctx.dtype == DType::BF16 && T > 0 && (T <= fused_rows || batch)) {
                     follow.norm = following;

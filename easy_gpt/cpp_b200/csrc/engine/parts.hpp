@@ -204,7 +204,7 @@ public:
         return out;
     }
 
-    // The same for steps of 17 to 64 tokens (gemm_batch.cu), of prepared rows (norm) or, into the residual, of plain ones
+    // The same for the steps that plans::batch_step takes (gemm_batch.cu), of prepared rows (norm) or, into the residual, of plain ones
     bool batch_takes(int epilogue, int head_dim) const { return dtype == DType::BF16 && eg_gemm_batch_takes(epilogue, out_features, in_features, head_dim) > 0; }
     void batch(const StepContext& ctx, int epilogue, int M, const Rows* x, const NormInFront* norm, void* out, long long ldo, const SkinnyRope* rope,
                const float* rotations, float* follow_residual, const float* follow_gain, void* xn_out, float* ss_out) const {
@@ -218,7 +218,7 @@ public:
 
     // whether with_following_norm can run for this input (the decode kernel takes it)
     bool takes_following_norm(const Rows& x) const {
-        if (plans::batch_tokens(dtype, x.rows)) return batch_takes(plans::EPI_RESID_NORM, 0) && aligned(x);
+        if (x.rows > plans::SKINNY_MAX_TOKENS) return x.rows <= plans::BATCH_MAX_TOKENS && batch_takes(plans::EPI_RESID_NORM, 0) && aligned(x);
         return dtype == DType::BF16 && plans::gemm_skinny_takes(dtype, x.rows, in_features) && x.rows <= plans::FUSED_NORM_MAX_TOKENS && aligned(x);
     }
     // The product, the add to the residual and the preparation of the norm that follows, in one kernel:

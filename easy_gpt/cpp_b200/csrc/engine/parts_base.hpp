@@ -269,7 +269,8 @@ public:
 };
 
 // Left by a part in place of its delta when it took a FollowingNorm over: the residual already holds the sum v;
-// rows is (compute dtype) gain * v and ss_parts float32 [parts, padded T] the partial sums of v^2 per token.
+// rows is (compute dtype) gain * v and ss_parts float32 the partial sums of v^2 per token, [parts, padded T] in steps of up to
+// plans::SKINNY_MAX_TOKENS tokens and [T, parts] in larger ones (each product reads what the product of the same step wrote).
 struct PreNormed {
     const Norm* norm = nullptr;
     void* rows = nullptr;
@@ -460,7 +461,7 @@ public:
     Mixer(const Params& params, const std::string& prefix, std::shared_ptr<PositionEncoding> position) : Part(params, prefix), position(std::move(position)) {}
     virtual bool accepts_pending_norm() const { return false; }
     virtual bool fuses_following_norm() const { return false; }
-    // whether it takes prepared rows in steps of 17 to 64 tokens too; writes: it writes its cache
+    // whether it takes prepared rows in the steps that plans::batch_step takes too; writes: it writes its cache
     virtual bool takes_prepared_batch(bool /*writes*/) const { return false; }
     virtual CacheNeed cache_need() const { return CacheNeed(); }
     // x [T, hidden] normalised input -> delta [T, hidden], both in ctx.dtype

@@ -145,9 +145,25 @@ inline SkinnyPlan skinny_plan(int n_rows, int in_features, int head_dim = 0) {
 inline bool gemm_skinny_takes(DType dtype, int tokens, int in_features) {
     return dtype == DType::BF16 && tokens > 0 && tokens <= SKINNY_MAX_TOKENS && in_features % 16 == 0;
 }
-// Steps of 17 to 64 tokens: rows that a product has prepared go from product to product (gemm_batch.cu) where the parts can say so.
+// Steps of 17 to 64 tokens whose rows go from product to product prepared (gemm_batch.cu), where the parts can say so; elsewhere the library's
+// products are as fast or faster.
+//   up to 32 tokens  decode steps of widths up to 1,536, others (prompts, and portions beside decoded tokens) up to 1,024; all from 3,584 on
+//   up to 64         decode steps of widths up to 896: a tie on the whole, and the library's steps were the same from run to run there less often
+// (us a step on the device, library / gemm_batch.  Decode steps of 17 / 24 / 32 requests, 300 keys: width 512, 8 layers, 228 234 235 / 195 198 199; 896,
+// 24 layers, 895 893 883 / 753 754 756; 1,024 with 16 heads of 64, 8 layers, 309 316 328 / 282 287 286; 1,536, 14 layers, 714 717 796 / 663 669 694; 2,048
+// with 16 heads of 128 and 5,632 wide, 416 418 430 / 427 421 425, and 11,008 wide 521 523 517 / 542 544 549; 2,560, 508 508 520 / 485 493 565; 3,072,
+// 470 471 475 / 447 466 484; 4,096, 604 605 607 / 541 553 561; 3,584 with 18,944 wide, where gate and up stay with the library, 60 keys, 738 739 741 / 714 715
+// 738.  Prompts of so many tokens: 512, 216 217 216 / 207 204 205; 896, 865 871 857 / 819 825 826;
+// 1,024, 281 284 285 / 280 268 271; 1,536, 682 682 764 / 713 721 746; 3,584, 859 738 739 / 838
+// 739 727; 4,096, 564 569 568 / 527 528 531.  33 / 48 / 64 requests: 896, 60 keys, 867 874 861 /
+// 891 897 903; 300, 906 914 902 / 895 904 931; 530, 933 957 986 / 908 922 950; the same with a head of 151,936 rows, served, 60 keys, 953 to 957, 963 to 1,050 and 946
+// to 1,046 / 946 954 986; 530, 1,021 to 1,128, 1,050 to 1,133 and 1,073 to 1,168 / 969 990 1,027; 512, 530 keys, 267 279 289 / 248 248 263; 1,024, 300 keys, 341
+// 348 361 / 362 369 380; 530, 378 386 399 / 435 445 437; 1,536, 530 keys, 826 832 841 / 906 919 979.)
 constexpr int BATCH_MAX_TOKENS = 64;
-inline bool batch_tokens(DType dtype, int tokens) { return dtype == DType::BF16 && tokens > SKINNY_MAX_TOKENS && tokens <= BATCH_MAX_TOKENS; }
+inline bool batch_step(DType dtype, int tokens, int width, bool all_decode) {
+    if (dtype != DType::BF16 || tokens <= SKINNY_MAX_TOKENS || tokens > BATCH_MAX_TOKENS) return false;
+    return tokens <= 32 ? width <= (all_decode ? 1536 : 1024) || width >= 3584 : all_decode && width <= 896;
+}
 inline int skinny_padded_tokens(int tokens) { return tokens <= 8 ? 8 : tokens <= 16 ? 16 : tokens <= 32 ? 32 : 64; }
 
 // How much of the feed-forward's first matrix the output projection in front of it asks the L2 for: what arrives while the

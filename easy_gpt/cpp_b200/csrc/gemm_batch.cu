@@ -13,9 +13,11 @@
 //   epilogues a thread has a token: into the residual with the next norm's preparation, SwiGLU of interleaved rows, or bias,
 //             rotation and cache write (a tile is a head).
 //
-// Bound by the chain of latencies behind the wait (x, the products, the exchange) and by the weights' stream; 14 to 152 column
-// tiles times CS give 50 to 150 CTAs, two of which share an SM.  (Measured: a step of 64 requests at 300 keys of the 0.5B sizes 1,038 us with
-// the library's products, 987 with the first form of these; 64 requests of 500 tokens served, 117 and 106 ms.)  Every wait is bounded.
+// Bound by the chain of latencies behind the wait (x, the products, the exchange) and by the weights' stream.  A product has one wave of
+// CTAs, two of which share an SM: up to 296 of them (gemm_batch_plan.h; at the 0.5B sizes 56 to 152).  Every column tile fetches all of x, as
+// many bytes as its weights at 64 tokens, and of the MMA's 128 rows as many are of use as there are tokens: with more than 32 tokens the library
+// is faster at most sizes, and so it is at larger widths (plans.hpp has the lines and the figures; a decode step of 32 requests at 300 keys of
+// the 0.5B sizes 883 us with the library's products, 756 with these).  Every wait is bounded.
 #define EG_NEEDS_TENSOR_MAPS
 #include "gemm_skinny.cuh"
 #include "gemm_batch_plan.h"
@@ -434,7 +436,8 @@ EG_API int eg_gemm_batch_takes(int epilogue, int N, int K, int head_dim) {
     return kind == batch_plan::INTO_RESIDUAL ? N / (c.columns / c.split) : 1;
 }
 
-// One product of a decode chain for M of 17 to 64 tokens.  epilogue 2 (SwiGLU of interleaved gate and up rows, out [M, N / 2]) and 3 (bias,
+// One product of a decode chain for M of 17 to 64 tokens.  W is read ahead, while the kernel in front still runs: nothing in the stream may
+// write it.  epilogue 2 (SwiGLU of interleaved gate and up rows, out [M, N / 2]) and 3 (bias,
 // rotation by `rotations` [M, head_dim / 2] cosines and sines, cache write; queries to out) read prepared rows x [M, K] with ss_in [M, ss_parts]
 // partial sums of squares; epilogue 4 (resid += x W^T + bias, xn = gain * resid, ss_out [M, parts] partial sums of squares of resid) reads
 // plain rows x [M, ldx].

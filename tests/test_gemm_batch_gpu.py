@@ -38,14 +38,16 @@ def off(got, want):
     return float((got.double() - want).norm() / want.norm())
 
 
-def run(epilogue, M, N, K, rng, heads, with_bias):
-    """(what the kernel gave, the same in float64)"""
+def run(epilogue, M, N, K, rng, heads, with_bias, scale=1.0, pad=0, prefetch=0):
+    """(what the kernel gave, the same in float64); scale: of the partial sums of squares; pad: what a row of x is longer than K; prefetch: bytes
+    that the L2 is asked for"""
     import torch
 
     lib = library()
     f32 = lambda *s: torch.from_numpy(rng.standard_normal(s).astype(np.float32)).cuda()  # noqa: E731
-    W, x = bf16(rng, N, K).cuda(), bf16(rng, M, K).cuda()
+    W, x = bf16(rng, N, K).cuda(), bf16(rng, M, K + pad).cuda()[:, :K]
     bias = f32(N) if with_bias else None
+    soon = torch.empty(max(prefetch, 1), device="cuda", dtype=torch.uint8) if prefetch else None
     status = torch.zeros(1, dtype=torch.int32, device="cuda")
     y = x.double() @ W.double().T
     empty = lambda *s, t=torch.bfloat16: torch.full(s, float("nan"), device="cuda", dtype=t)  # noqa: E731
@@ -55,7 +57,7 @@ def run(epilogue, M, N, K, rng, heads, with_bias):
         resid, gain = f32(M, N) * 30, f32(N)
         a.update(resid=resid.clone(), gain=gain, xn=empty(M, N), ss=empty(M, parts, t=torch.float32))
     else:
-        ss = f32(M, 24).square()
+        ss = f32(M, 24).square() * scale
         a["ssi"] = ss
         y *= 1.0 / torch.sqrt(ss.double().sum(1, keepdim=True) / K + 1e-6)
     if with_bias:
@@ -70,9 +72,9 @@ def run(epilogue, M, N, K, rng, heads, with_bias):
         cache = torch.full((5, 2, G, 16, hd), 7.0, device="cuda", dtype=torch.bfloat16)
         a.update(out=empty(M, H * hd), ldo=H * hd, rot=rot, slots=slots.cuda(), ps=16, pst=2 * G * 16 * hd, hst=16 * hd, pool=80, k=cache, v=cache[:, 1])
     ptr = lambda t: None if t is None else t.data_ptr()  # noqa: E731
-    rc = lib.eg_gemm_batch(torch.cuda.current_stream().cuda_stream, epilogue, 2, ptr(W), K, ptr(bias), M, N, K, ptr(x), K, 1e-6, ptr(a["ssi"]), 24 if a["ssi"] is not None else 0,
+    rc = lib.eg_gemm_batch(torch.cuda.current_stream().cuda_stream, epilogue, 2, ptr(W), K, ptr(bias), M, N, K, ptr(x), K + pad, 1e-6, ptr(a["ssi"]), 24 if a["ssi"] is not None else 0,
                            ptr(a["out"]), a["ldo"], *heads, ptr(a["rot"]), ptr(a["slots"]), ptr(a["k"]), ptr(a["v"]), a["ps"], a["pst"], a["hst"], a["pool"], ptr(a["resid"]),
-                           ptr(a["gain"]), ptr(a["xn"]), ptr(a["ss"]), None, 0, ptr(status))
+                           ptr(a["gain"]), ptr(a["xn"]), ptr(a["ss"]), ptr(soon), prefetch, ptr(status))
     torch.cuda.synchronize()
     assert rc == 0 and int(status[0]) == 0
     if epilogue == SWIGLU:
@@ -134,3 +136,23 @@ def test_a_chain_of_products_whatever_the_dependents_wait_for(M, N, K):
     assert off(got[0][0] - resid, 24 * step.double()) < 2.0 ** -8
     for other in got[1:]:
         assert all(bool((a == b).all()) for a, b in zip(got[0], other))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("M", [17, 32, 33, 64])
+@pytest.mark.parametrize("epilogue,N,K,heads", [(QKV, 512, 512, (2, 1, 128)), (QKV, 1152, 896, (14, 2, 64)), (QKV, 2048, 1536, (12, 2, 128)), (SWIGLU, 9728, 896, (0, 0, 0)),
+                                                (SWIGLU, 128, 64, (0, 0, 0)), (RESID, 896, 4864, (0, 0, 0)), (RESID, 256, 320, (0, 0, 0))])
+def test_products_value_by_value(epilogue, N, K, heads, M):
+    """Products of order one, so that gates are neither open nor shut, every value by itself: one rounding to bfloat16 (eight bits: at most 2^-8 of
+    it; two of them for xn, its own and its term's, which the gain multiplies), and what float32 sums of K products lose, 2^-24 sqrt(K) of the largest, at most 1e-4 of the usual value.  Heads
+    of 128 in clusters of four and of eight; rows of x longer than K, and with weights asked for ahead, where the epilogue takes them."""
+    plain_rows = epilogue == RESID
+    got, want = run(epilogue, M, N, K, np.random.default_rng([epilogue, M, N, 5]), heads, M % 2 == 0, scale=K * K / 24, pad=64 if plain_rows else 0,
+                    prefetch=100_000 if plain_rows else 0)
+    for i, (g, w) in enumerate(zip(got, want)):
+        slack = 2.0 ** -8 * w.abs() + 1e-4 * float(w.square().mean().sqrt())
+        if plain_rows and i == 1:                                # xn: the gain is normal, 4.5 at most
+            slack = slack + 2.0 ** -8 * 4.5 * want[0].abs()
+        if plain_rows and i == 2:
+            slack = 1e-5 * w
+        assert bool(((g.double() - w).abs() <= slack).all()), (i, float(((g.double() - w).abs() - slack).max()))
