@@ -1,9 +1,10 @@
 // Matrix products for decode steps (1..64 tokens): y[m, n] = sum_k x[m, k] W[n, k].
 //
 // The kernel of this file is register-fed; up to 16 tokens gemm_stream.cu takes the products whose rows need no add + norm
-// here (all but a step's first), and this one the rest: 17 to 64 tokens, the add + norm prologue, heads that are no multiple
+// here (all but a step's first), and this one the rest: the add + norm prologue, heads that are no multiple
 // of 32, residuals whose partial sums are asked for by larger groups of rows, and what gemm_stream_plan.h does not take: x of
-// 16 tokens or clusters that do not fit (the 7B down product, 3,584 x 18,944, among them).
+// 16 tokens or clusters that do not fit (the 7B down product, 3,584 x 18,944, among them).  (17 to 64 tokens go elsewhere in the engine, to
+// gemm_batch.cu or the library, and come here only by themselves.)
 //
 // With so few tokens the product is a stream of the weights from HBM, so the
 // kernel is built around that stream.  The roles of the MMA are swapped: 16 weight

@@ -1,4 +1,4 @@
-"""The decode attention over short contexts (one CTA of eight warps walks them) and one key tile beyond, against plain attention in float64:
+"""The decode attention over short contexts (one CTA of eight or sixteen warps walks them) and one key tile beyond, against plain attention in float64:
 contexts at the edges of key tiles, rounds and of the form itself, whatever number of splits was asked for, windows, fresh keys, and tokens
 without a list of their sequences (token i is sequence i's)."""
 import math
@@ -14,7 +14,7 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("heads", [(14, 2, 64), (12, 2, 128), (4, 4, 32), (16, 1, 64)])
 @pytest.mark.parametrize("window", [0, 100])
 def test_short_contexts(heads, width, splits, window):
-    """P and the result are rounded to bfloat16: 2^-8 of the values' norm, as the other tests of this kernel."""
+    """P and the result are rounded to bfloat16, each by up to 2^-8 of a value: 2^-7 of the norm, as the other tests of this kernel."""
     import torch
 
     from easy_gpt.cpp_b200 import kernels

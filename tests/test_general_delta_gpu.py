@@ -1,5 +1,5 @@
 """The generalised delta rule's kernels by themselves, against the recurrence in float64: prompts whose entries go in chunks of 16
-tokens (heads of 64, 32 tokens an entry on average) and those next to that border, entries that end anywhere in a chunk, states that
+tokens (heads of 64, 32 tokens an entry on average, one of 48 among more than two) and those next to that border, entries that end anywhere in a chunk, states that
 are there already, decays next to one and far from it."""
 import ctypes
 
